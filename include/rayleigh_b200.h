@@ -629,8 +629,8 @@ int ra_radius(const ra_ctx* ctx, double* radius);
 int ra_costheta(const ra_ctx* ctx, double* costheta);
 
 /* Kernel choices of the tunable stages (the autotuner's knobs):
- *   "physics"   physical-space kernel: 1 every FFT pass in shared memory
- *               (n_theta <= 768); 0 the last (radix-3) pass and the
+ *   "physics"   physical-space kernel: 1 on (theta, pi - theta) row pairs, both
+ *               rows in one complex FFT (n_theta <= 768); 0 the last (radix-3) pass and the
  *               nonlinear terms in registers, two CTAs per SM, 2 the same
  *               with one CTA per SM (n_theta 384, 768, 1536; the only
  *               kernel at 1536)

@@ -1,23 +1,6 @@
-// Physical-space stage, fused per (r, theta) row:
-//   Phi_Derivatives           (Sphere_Physical_Space.F90:745-759) in the spectrum load,
-//   fft_to_physical  (c2r)    (Fourier_Transform.F90:142-183), 14 fields,
-//   sintheta_div + NL terms   (Sphere_Physical_Space.F90:98-224, 303-700),
-//   Find_MyMinDT (CFL max)    (:784-813),
-//   fft_to_spectral (r2c)     (Fourier_Transform.F90:100-140), 4 fields,
-//   equatorial fold of PtS    (Legendre_Transforms.F90:1109-1122),
-// reading the inverse Legendre output p2a[theta_h][m][par][r][f][re/im] (E, O) and
-// writing the folded p2b[m][par][theta_h][r][f][re/im] for m <= l_max.  The
-// reference materialises the packed (n_phi+2, r, theta, f) buffers p3a/p3b
-// between these steps; here the 18 phi rows of one (r, theta) point never
-// leave the SM.
-//
-// One CTA (384 threads, two per SM) handles one row; the rows theta and
-// pi - theta are the two CTAs of a cluster, which fold their spectra through
-// distributed shared memory.  The 14 input fields go through the FFT in
-// batches of four, four, four and two; the four nonlinear outputs accumulate
-// in shared memory (each thread owns its points), the velocity in registers,
-// the row's radial and colatitude factors in shared memory.  The same c2r
-// serves the output-iteration diagnostics (kinetic energy, shell slices).
+// phi transforms per (r, theta) row: the diagnostics' row synthesis, the unit FFTs, and the
+// physical-space stage at n_theta = 1536 (and on request at 384 and 768) with the last FFT pass
+// in registers.  The step's physical-space stage runs on row pairs (k_physics_pair.cu).
 //
 // FFT: a real length-2N transform through one complex length-N transform
 // (N = n_theta = 2^a 3^b), in place in shared memory: decimation in frequency
@@ -35,6 +18,7 @@
 
 #include <cooperative_groups.h>
 
+#include "phi_fft.cuh"
 #include "ra_internal.h"
 
 namespace ra {
@@ -44,13 +28,6 @@ struct FFTPlan {
     int npass;
     int radix[16];
 };
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 
 // exp(sign * 2 pi i e / N) from wr[k] = exp(2 pi i k / (2N)), k < N
 __device__ __forceinline__ double2 twiddle(const double2* wr, int N, int e, int sign) {
@@ -70,85 +47,6 @@ __device__ __forceinline__ double2 twiddle_g(const double2* __restrict__ wr, int
     }
     if (sign < 0) w.y = -w.y;
     return w;
-}
-
-__device__ __forceinline__ void dft4(double2& u0, double2& u1, double2& u2, double2& u3, int sign) {
-    const double2 t0 = cadd(u0, u2), t1 = csub(u0, u2);
-    const double2 t2 = cadd(u1, u3), d = csub(u1, u3);
-    // w = sign * i : w * (x + i y) = sign * (-y + i x)
-    const double2 wd = make_double2(-sign * d.y, sign * d.x);
-    u0 = cadd(t0, t2);
-    u2 = csub(t0, t2);
-    u1 = cadd(t1, wd);
-    u3 = csub(t1, wd);
-}
-
-__device__ __forceinline__ void dft_small(int R, double2* u, int sign) {
-    if (R == 2) {
-        const double2 a = u[0], b = u[1];
-        u[0] = cadd(a, b);
-        u[1] = csub(a, b);
-    } else if (R == 4) {
-        dft4(u[0], u[1], u[2], u[3], sign);
-    } else if (R == 16) {
-        // 16 = 4 x 4: DFT-4 over the elements q + 4p, twiddle w16^(q k1), DFT-4 over q;
-        // output k1 + 4 k2
-        const double C1 = 0.92387953251128675613, S1 = 0.38268343236508977173;   // cos, sin pi/8
-        const double H = 0.70710678118654752440;                                  // cos pi/4
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dft4(u[q], u[q + 4], u[q + 8], u[q + 12], sign);
-        // element (q, k1) sits at u[q + 4 k1]; w16^e = (cos, sign sin)(2 pi e / 16)
-        auto tw16 = [&](double2 a, int e) -> double2 {
-            double c, sn;
-            switch (e) {
-                case 1: c = C1; sn = S1; break;
-                case 2: c = H; sn = H; break;
-                case 3: c = S1; sn = C1; break;
-                case 4: c = 0.0; sn = 1.0; break;
-                case 6: c = -H; sn = H; break;
-                case 9: c = -C1; sn = -S1; break;
-                default: c = 1.0; sn = 0.0; break;
-            }
-            sn *= sign;
-            return make_double2(a.x * c - a.y * sn, a.x * sn + a.y * c);
-        };
-#pragma unroll
-        for (int q = 1; q < 4; ++q)
-#pragma unroll
-            for (int k1 = 1; k1 < 4; ++k1) u[q + 4 * k1] = tw16(u[q + 4 * k1], q * k1);
-        double2 v[16];
-#pragma unroll
-        for (int k1 = 0; k1 < 4; ++k1) {
-            double2 a0 = u[0 + 4 * k1], a1 = u[1 + 4 * k1], a2 = u[2 + 4 * k1], a3 = u[3 + 4 * k1];
-            dft4(a0, a1, a2, a3, sign);
-            v[k1 + 0] = a0;
-            v[k1 + 4] = a1;
-            v[k1 + 8] = a2;
-            v[k1 + 12] = a3;
-        }
-#pragma unroll
-        for (int k = 0; k < 16; ++k) u[k] = v[k];
-    } else if (R == 8) {
-        const double H = 0.70710678118654752440;   // sqrt(2)/2
-        double2 a0 = cadd(u[0], u[4]), a1 = cadd(u[1], u[5]), a2 = cadd(u[2], u[6]), a3 = cadd(u[3], u[7]);
-        double2 b0 = csub(u[0], u[4]), b1 = csub(u[1], u[5]), b2 = csub(u[2], u[6]), b3 = csub(u[3], u[7]);
-        // b_j *= exp(sign i pi j / 4)
-        b1 = make_double2(H * (b1.x - sign * b1.y), H * (b1.y + sign * b1.x));
-        b2 = make_double2(-sign * b2.y, sign * b2.x);
-        b3 = make_double2(H * (-b3.x - sign * b3.y), H * (-b3.y + sign * b3.x));
-        dft4(a0, a1, a2, a3, sign);
-        dft4(b0, b1, b2, b3, sign);
-        u[0] = a0; u[2] = a1; u[4] = a2; u[6] = a3;
-        u[1] = b0; u[3] = b1; u[5] = b2; u[7] = b3;
-    } else {  // R == 3
-        const double S3 = 0.86602540378443864676;
-        const double2 t = cadd(u[1], u[2]), d = csub(u[1], u[2]);
-        const double2 a = make_double2(u[0].x - 0.5 * t.x, u[0].y - 0.5 * t.y);
-        const double2 sd = make_double2(-sign * S3 * d.y, sign * S3 * d.x);
-        u[0] = cadd(u[0], t);
-        u[1] = cadd(a, sd);
-        u[2] = csub(a, sd);
-    }
 }
 
 // Runs nb independent FFTs of length N stored at a + b*N (b < nb), scratch at
@@ -221,27 +119,9 @@ __device__ __forceinline__ int SW(int i) { return i; }
 // eight different bank groups per quarter warp (n is a multiple of 8).
 __host__ __device__ constexpr int fstride(int n) { return n + 2; }
 
-struct PhysParams {
-    const double* p2a;
-    double* p2b;
-    const double* radial;   // packed radial profiles
-    const double* trig;     // [4][nth]: cos, sin, csc, cot
-    const double2* wr;      // [nth] exp(2 pi i k / n_phi)
-    const double2* twp;     // per-pass FFT twiddles (ip_tw_off; one load per butterfly, twiddle_apply)
-    unsigned long long* cfl;
-    int L, nth, nr, ncola, ncolb;
-    double coriolis;
-    int rotation;
-    double llmax;
-    int nfa, nfb;           // fields per radius of p2a / p2b
-    double lorentz;         // Lorentz_Coeff (magnetism)
-};
-
 // One CTA = one (theta, r) row; the rows theta and pi - theta of a pair form a
 // 2-CTA cluster that folds its spectra through distributed shared memory.
 constexpr int ROW_THREADS = 384;
-enum { RC_RAD, RC_ORAD, RC_RHO, RC_DLNRHO, RC_DR, RC_CS, RC_SN, RC_CSC, RC_COT, RC_COR, RC_C2R, RC_HSF, RC_VH, RC_OH,
-       RC_COUNT };
 constexpr int FB = 4;   // fields per batched FFT
 
 // Shared memory of a row CTA (double2 units): one in-place FFT buffer of FB
@@ -272,32 +152,6 @@ __host__ __device__ constexpr int ip_tw_off(int n, int ps) {
     return o;
 }
 __host__ __device__ constexpr int ip_tw_size(int n) { return ip_tw_off(n, npass_of(n)); }
-
-// u[k] *= w^k, k = 1 .. R-1, for the butterfly's one table twiddle w: the
-// powers are complex products (at most three deep, a few units in the last
-// place) formed in the order they are used, w^2 = w w, w^3 = w^2 w,
-// w^4 = w^2 w^2, w^5 = w^4 w, w^6 = w^4 w^2, w^7 = w^4 w^3, so that no more
-// than four of them are live next to the butterfly's R values.
-template <int R>
-__device__ __forceinline__ void twiddle_apply(double2 (&u)[R], double2 w1) {
-    static_assert(R == 2 || R == 3 || R == 4 || R == 8, "radix");
-    u[1] = cmul(u[1], w1);
-    if constexpr (R >= 3) {
-        const double2 w2 = cmul(w1, w1);
-        u[2] = cmul(u[2], w2);
-        if constexpr (R >= 4) {
-            const double2 w3 = cmul(w2, w1);
-            u[3] = cmul(u[3], w3);
-            if constexpr (R == 8) {
-                const double2 w4 = cmul(w2, w2);
-                u[4] = cmul(u[4], w4);
-                u[5] = cmul(u[5], cmul(w4, w1));
-                u[6] = cmul(u[6], cmul(w4, w2));
-                u[7] = cmul(u[7], cmul(w4, w3));
-            }
-        }
-    }
-}
 
 // Butterfly g of a pass -> (field f, block b, offset j).  The plain order runs
 // over (f, b, j).  A 16-byte shared access is served in 8-lane phases, one
@@ -561,385 +415,6 @@ __device__ __forceinline__ void r2c_finish(double2* a, int nf, int L, const doub
     }
 }
 
-template <int NTH, bool MAG, bool HEAT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROW_THREADS, 2) physics_kernel(PhysParams P) {
-    constexpr int N = NTH;
-    constexpr int FS = fstride(N);
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double2* sm = reinterpret_cast<double2*>(smem_raw);
-    double2* acc = sm + RowSmem<N>::ACC;
-    __shared__ double red[ROW_THREADS / 32];
-    const int t = threadIdx.x;
-    const int h = (int)cluster.block_rank();        // 0: theta (south half), 1: pi - theta
-    const int nr = P.nr;
-    const int pair = blockIdx.x >> 1;
-    const int r = pair % nr;
-    const int thh = pair / nr;
-    const int th = h ? (N - 1 - thh) : thh;
-    const double* rowbase = P.p2a + (long)thh * (2L * P.L * P.ncola) + (long)r * (2 * P.nfa);
-    // The row's radial and colatitude factors live in shared memory and are read
-    // where they are used, so that they hold no registers across the FFTs.
-    __shared__ double rowc[RC_COUNT];
-    if (t == 0) {
-        const double csc = P.trig[2 * N + th], orad = P.radial[R_OVER_R * nr + r];
-        rowc[RC_RAD] = P.radial[R_RADIUS * nr + r];
-        rowc[RC_ORAD] = orad;
-        rowc[RC_RHO] = P.radial[R_DENSITY * nr + r];
-        rowc[RC_DLNRHO] = P.radial[R_DLNRHO * nr + r];
-        rowc[RC_DR] = P.radial[R_DELTA_R * nr + r];
-        rowc[RC_CS] = P.trig[th];
-        rowc[RC_SN] = P.trig[N + th];
-        rowc[RC_CSC] = csc;
-        rowc[RC_COT] = P.trig[3 * N + th];
-        rowc[RC_COR] = P.rotation ? P.coriolis : 0.0;
-        rowc[RC_C2R] = csc * csc * orad;
-        rowc[RC_HSF] = 0.5 * (P.radial[R_DENSITY * nr + r] * P.radial[R_RADIUS * nr + r] * csc);
-        rowc[RC_VH] = P.radial[R_VISC_HEAT * nr + r];
-        rowc[RC_OH] = P.radial[R_OHM_HEAT * nr + r];
-    }   // read after row_c2r's first barrier
-
-    double2 vr[ZPT], vt[ZPT], vp[ZPT];
-    double2 y[FB][ZPT];
-    auto acc_at = [&](int f, int q) -> double2& { return acc[SW(f * FS + t + q * ROW_THREADS)]; };
-    auto live = [&](int q) { return t + q * ROW_THREADS < N; };
-    if constexpr (HEAT) {
-        // The anelastic form: the same terms, with the viscous heating
-        // (Compute_Viscous_Heating, Sphere_Physical_Space.F90:337-443) in T's accumulator.
-        // Its strain-rate components are products across fields, so the batches are
-        // regrouped for each component to complete inside one batch:
-        //   H1: v_r, v_theta, v_phi
-        //   H2: dv_r/dtheta, dv_r/dphi, dv_theta/dr, dv_phi/dr  -> 2 e_r_theta, 2 e_r_phi
-        //   H3: dv_phi/dphi, omega_r, dv_theta/dphi, dv_r/dr    -> e_rr, e_theta_theta,
-        //       e_phi_phi, 2 e_phi_theta (dv_theta/dtheta, dv_phi/dtheta as :226-248 form them)
-        //   H4: dT/dr, dT/dtheta, dT/dphi
-        {
-            const int fo[3] = {A_VR, A_VT, A_VP};
-            const bool dp[3] = {false, false, false};
-            row_c2r<N, 3, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], dlnrho = rowc[RC_DLNRHO];
-            const double cs = rowc[RC_CS], sn = rowc[RC_SN], csc = rowc[RC_CSC], cot = rowc[RC_COT], cor = rowc[RC_COR];
-#pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                vr[q] = y[0][q];
-                vt[q] = make_double2(y[1][q].x * csc, y[1][q].y * csc);
-                vp[q] = make_double2(y[2][q].x * csc, y[2][q].y * csc);
-                auto w0 = [&](double b, double c) { return rho * (rad * b * b + rad * c * c + cor * sn * rad * rad * c); };
-                auto p0 = [&](double a, double b, double c) {
-                    return -b * b * cot * orad - b * a * orad - b * a * dlnrho - c * c * cot * orad - cor * cs * c;
-                };
-                auto z0 = [&](double a, double b, double c) { return c * a * orad + cor * (cs * b + sn * a); };
-                if (live(q)) {
-                    acc_at(0, q) = make_double2(w0(vt[q].x, vp[q].x), w0(vt[q].y, vp[q].y));
-                    acc_at(1, q) = make_double2(p0(vr[q].x, vt[q].x, vp[q].x), p0(vr[q].y, vt[q].y, vp[q].y));
-                    acc_at(3, q) = make_double2(z0(vr[q].x, vt[q].x, vp[q].x), z0(vr[q].y, vt[q].y, vp[q].y));
-                }
-            }
-        }
-        {
-            const int fo[4] = {A_DVRDT, A_VR, A_DVTDR, A_DVPDR};
-            const bool dp[4] = {false, true, false, false};
-            row_c2r<N, 4, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], csc = rowc[RC_CSC];
-            const double dlnrho = rowc[RC_DLNRHO], vh = rowc[RC_VH];
-#pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                double2& w = acc_at(0, q);
-                double2& pp = acc_at(1, q);
-                double2& z = acc_at(3, q);
-                // a = sin(theta) dv_r/dtheta, b = dv_r/dphi, c = sin(theta) dv_theta/dr, d = sin(theta) dv_phi/dr
-                auto terms = [&](double a, double b, double c, double d, double vrr, double vtt, double vpp, double& wv,
-                                 double& pv, double& zv) {
-                    wv += -rho * rad * vtt * a * csc - rho * rad * csc * vpp * b;
-                    pv += vrr * c * csc;
-                    zv += vrr * d * csc;
-                    const double erth = (a * csc - vtt) * orad + c * csc;   // 2 e_r_theta
-                    const double erph = (b * csc - vpp) * orad + d * csc;   // 2 e_r_phi
-                    const double dv = -vrr * dlnrho;                        // div u
-                    return vh * (erth * erth * 0.5 + erph * erph * 0.5 - dv * dv * (1.0 / 3.0));
-                };
-                const double hx = terms(y[0][q].x, y[1][q].x, y[2][q].x, y[3][q].x, vr[q].x, vt[q].x, vp[q].x, w.x,
-                                        pp.x, z.x);
-                const double hy = terms(y[0][q].y, y[1][q].y, y[2][q].y, y[3][q].y, vr[q].y, vt[q].y, vp[q].y, w.y,
-                                        pp.y, z.y);
-                acc_at(2, q) = make_double2(hx, hy);
-            }
-        }
-        {
-            const int fo[4] = {A_VP, A_OMR, A_VT, A_DVRDR};
-            const bool dp[4] = {true, false, true, false};
-            row_c2r<N, 4, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], csc = rowc[RC_CSC];
-            const double cot = rowc[RC_COT], c2r = rowc[RC_C2R], dlnrho = rowc[RC_DLNRHO], vh = rowc[RC_VH];
-            const double csc2 = csc * csc;
-#pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                double2& w = acc_at(0, q);
-                double2& pp = acc_at(1, q);
-                double2& tt = acc_at(2, q);
-                double2& z = acc_at(3, q);
-                // a = sin(theta) dv_phi/dphi, b = omega_r, c = sin(theta) dv_theta/dphi, x = dv_r/dr
-                auto terms = [&](double a, double b, double c, double x, double vrr, double vtt, double vpp, double& wv,
-                                 double& pv, double& zv) {
-                    wv += -rho * rad * rad * vrr * x;
-                    pv += -vtt * x + vpp * c * c2r - vtt * a * c2r;
-                    zv += vtt * c * c2r + vpp * a * c2r + vtt * b;
-                    const double dvtdt = -vrr * (rad * dlnrho + 2.0) - rad * x - vtt * cot - a * csc2;
-                    const double dvpdt = rad * b + c * csc2 - vpp * cot;
-                    const double eff = (a * csc2 + vrr + vtt * cot) * orad;     // e_phi_phi
-                    const double ett = (dvtdt + vrr) * orad;                    // e_theta_theta
-                    const double eph = (dvpdt + c * csc2 - vpp * cot) * orad;   // 2 e_phi_theta
-                    return vh * (x * x + eff * eff + ett * ett + eph * eph * 0.5);
-                };
-                tt.x += terms(y[0][q].x, y[1][q].x, y[2][q].x, y[3][q].x, vr[q].x, vt[q].x, vp[q].x, w.x, pp.x, z.x);
-                tt.y += terms(y[0][q].y, y[1][q].y, y[2][q].y, y[3][q].y, vr[q].y, vt[q].y, vp[q].y, w.y, pp.y, z.y);
-            }
-        }
-        {
-            const int fo[3] = {A_DTDR, A_DTDT, A_T};
-            const bool dp[3] = {false, false, true};
-            row_c2r<N, 3, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double csc = rowc[RC_CSC], orad = rowc[RC_ORAD];
-#pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                const double2 d = y[0][q], a = y[1][q], b = y[2][q];
-                double2& tt = acc_at(2, q);
-                tt.x += -vr[q].x * d.x - a.x * csc * vt[q].x * orad - vp[q].x * b.x * csc * orad;
-                tt.y += -vr[q].y * d.y - a.y * csc * vt[q].y * orad - vp[q].y * b.y * csc * orad;
-            }
-        }
-    } else {
-        // B1: v_r, v_theta, v_phi, dv_r/dr: the quadratic, Coriolis and radial-advection terms
-        {
-            const int fo[4] = {A_VR, A_VT, A_VP, A_DVRDR};
-            const bool dp[4] = {false, false, false, false};
-            row_c2r<N, 4, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], dlnrho = rowc[RC_DLNRHO];
-            const double cs = rowc[RC_CS], sn = rowc[RC_SN], csc = rowc[RC_CSC], cot = rowc[RC_COT], cor = rowc[RC_COR];
-    #pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                vr[q] = y[0][q];
-                vt[q] = y[1][q];
-                vp[q] = y[2][q];
-                vt[q].x *= csc;
-                vt[q].y *= csc;
-                vp[q].x *= csc;
-                vp[q].y *= csc;
-                const double2 x = y[3][q];
-                auto w0 = [&](double a, double b, double c, double xx) {
-                    return rho * (rad * b * b + rad * c * c + cor * sn * rad * rad * c) - rho * rad * rad * a * xx;
-                };
-                auto p0 = [&](double a, double b, double c, double xx) {
-                    return -b * b * cot * orad - b * a * orad - b * a * dlnrho - c * c * cot * orad - cor * cs * c - b * xx;
-                };
-                auto z0 = [&](double a, double b, double c) { return c * a * orad + cor * (cs * b + sn * a); };
-                if (live(q)) {
-                    acc_at(0, q) = make_double2(w0(vr[q].x, vt[q].x, vp[q].x, x.x), w0(vr[q].y, vt[q].y, vp[q].y, x.y));
-                    acc_at(1, q) = make_double2(p0(vr[q].x, vt[q].x, vp[q].x, x.x), p0(vr[q].y, vt[q].y, vp[q].y, x.y));
-                    acc_at(3, q) = make_double2(z0(vr[q].x, vt[q].x, vp[q].x), z0(vr[q].y, vt[q].y, vp[q].y));
-                }
-            }
-        }
-        // B2: dv_r/dtheta, dv_r/dphi, dv_theta/dr, dv_theta/dphi
-        {
-            const int fo[4] = {A_DVRDT, A_VR, A_DVTDR, A_VT};
-            const bool dp[4] = {false, true, false, true};
-            row_c2r<N, 4, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double rad = rowc[RC_RAD], rho = rowc[RC_RHO], csc = rowc[RC_CSC], c2r = rowc[RC_C2R];
-    #pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                const double2 a = y[0][q], b = y[1][q], c = y[2][q], d = y[3][q];
-                double2& w = acc_at(0, q);
-                double2& pp = acc_at(1, q);
-                double2& z = acc_at(3, q);
-                w.x += -rho * rad * vt[q].x * a.x * csc - rho * rad * csc * vp[q].x * b.x;
-                w.y += -rho * rad * vt[q].y * a.y * csc - rho * rad * csc * vp[q].y * b.y;
-                pp.x += vr[q].x * c.x * csc + vp[q].x * d.x * c2r;
-                pp.y += vr[q].y * c.y * csc + vp[q].y * d.y * c2r;
-                z.x += vt[q].x * d.x * c2r;
-                z.y += vt[q].y * d.y * c2r;
-            }
-        }
-        // B3: dv_phi/dr, dv_phi/dphi, omega_r, dT/dr (the T term's first part, written)
-        {
-            const int fo[4] = {A_DVPDR, A_VP, A_OMR, A_DTDR};
-            const bool dp[4] = {false, true, false, false};
-            row_c2r<N, 4, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double csc = rowc[RC_CSC], c2r = rowc[RC_C2R];
-    #pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                const double2 a = y[0][q], b = y[1][q], c = y[2][q], d = y[3][q];
-                double2& pp = acc_at(1, q);
-                double2& z = acc_at(3, q);
-                z.x += vr[q].x * a.x * csc + vp[q].x * b.x * c2r + vt[q].x * c.x;
-                z.y += vr[q].y * a.y * csc + vp[q].y * b.y * c2r + vt[q].y * c.y;
-                pp.x += -vt[q].x * b.x * c2r;
-                pp.y += -vt[q].y * b.y * c2r;
-                acc_at(2, q) = make_double2(-vr[q].x * d.x, -vr[q].y * d.y);
-            }
-        }
-        // B4: dT/dtheta, dT/dphi
-        {
-            const int fo[2] = {A_DTDT, A_T};
-            const bool dp[2] = {false, true};
-            row_c2r<N, 2, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double csc = rowc[RC_CSC], orad = rowc[RC_ORAD];
-    #pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                const double2 a = y[0][q], b = y[1][q];
-                double2& tt = acc_at(2, q);
-                tt.x += -a.x * csc * vt[q].x * orad - vp[q].x * b.x * csc * orad;
-                tt.y += -a.y * csc * vt[q].y * orad - vp[q].y * b.y * csc * orad;
-            }
-        }
-    }
-    // CFL (Find_MyMinDT); the rho r / sin(theta) factor of the P and Z terms is a
-    // row constant, applied to their spectra after the r2c (RC_HSF)
-    double cmax = 0.0;
-    const double orad = rowc[RC_ORAD], dr = rowc[RC_DR];
-    const double hfac = P.llmax * orad * orad, rfac = 1.0 / (dr * dr);
-#pragma unroll
-    for (int q = 0; q < ZPT; ++q) {
-        if (live(q)) {
-            cmax = fmax(cmax, (vt[q].x * vt[q].x + vp[q].x * vp[q].x) * hfac);
-            cmax = fmax(cmax, (vt[q].y * vt[q].y + vp[q].y * vp[q].y) * hfac);
-            cmax = fmax(cmax, vr[q].x * vr[q].x * rfac);
-            cmax = fmax(cmax, vr[q].y * vr[q].y * rfac);
-        }
-    }
-    if constexpr (MAG) {
-        // M1: B_r, B_theta, B_phi, (curl B)_r.  The EMF u x B (Compute_EMF,
-        // Sphere_Physical_Space.F90:534-581) replaces them in the FFT buffer and goes through
-        // its own r2c and fold into p2b fields B_EMFT, B_EMFR, B_EMFP; B stays in registers
-        // for the Lorentz force, which M2 ((curl B)_theta, (curl B)_phi) completes.
-        double2 br[ZPT], bt[ZPT], bp[ZPT], cbr[ZPT];
-        double2* buf = sm + RowSmem<N>::BUF;
-        {
-            const int fo[4] = {A_BR, A_BT, A_BP, A_CBR};
-            const bool dp[4] = {false, false, false, false};
-            row_c2r<N, 4, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double csc = rowc[RC_CSC], rad = rowc[RC_RAD], rho = rowc[RC_RHO];
-            // the Alfven speed (:798-806)
-            const double hfb = P.llmax * orad * orad / rho * P.lorentz, rfb = P.lorentz / (dr * dr * rho);
-#pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                br[q] = y[0][q];
-                bt[q] = make_double2(y[1][q].x * csc * orad, y[1][q].y * csc * orad);   // rsintheta_div
-                bp[q] = make_double2(y[2][q].x * csc * orad, y[2][q].y * csc * orad);
-                cbr[q] = y[3][q];
-                if (!live(q)) continue;
-                if constexpr (HEAT) {   // Compute_Ohmic_Heating (:446-466), the (curl B)_r part
-                    const double oh = rowc[RC_OH];
-                    acc_at(2, q).x += cbr[q].x * cbr[q].x * oh;
-                    acc_at(2, q).y += cbr[q].y * cbr[q].y * oh;
-                }
-                cmax = fmax(cmax, (bt[q].x * bt[q].x + bp[q].x * bp[q].x) * hfb);
-                cmax = fmax(cmax, (bt[q].y * bt[q].y + bp[q].y * bp[q].y) * hfb);
-                cmax = fmax(cmax, br[q].x * br[q].x * rfb);
-                cmax = fmax(cmax, br[q].y * br[q].y * rfb);
-                auto emft = [&](double a, double c, double b_r, double b_p) { return (-a * b_p + c * b_r) * csc * rad; };
-                auto emfr = [&](double b, double c, double b_t, double b_p) { return b * b_p - c * b_t; };
-                auto emfp = [&](double a, double b, double b_r, double b_t) { return (a * b_t - b * b_r) * csc * rad; };
-                const int n = t + q * ROW_THREADS;
-                buf[SW(0 * FS + n)] = make_double2(emft(vr[q].x, vp[q].x, br[q].x, bp[q].x),
-                                                   emft(vr[q].y, vp[q].y, br[q].y, bp[q].y));
-                buf[SW(1 * FS + n)] = make_double2(emfr(vt[q].x, vp[q].x, bt[q].x, bp[q].x),
-                                                   emfr(vt[q].y, vp[q].y, bt[q].y, bp[q].y));
-                buf[SW(2 * FS + n)] = make_double2(emfp(vr[q].x, vt[q].x, br[q].x, bt[q].x),
-                                                   emfp(vr[q].y, vt[q].y, br[q].y, bt[q].y));
-            }
-        }
-        __syncthreads();
-        fft_dit<N, 3, ROW_THREADS>(buf, P.twp, t);
-        r2c_finish<N>(buf, 3, P.L, P.wr, t, [](int) { return 0.5; });
-        cluster.sync();
-        {
-            const double2* peer = cluster.map_shared_rank(buf, h ^ 1);
-            const int L = P.L;
-            const long mstride = 2L * (P.nth / 2) * P.ncolb;
-            double* obase = P.p2b + (long)h * (P.nth / 2) * P.ncolb + (long)thh * P.ncolb + (long)r * (2 * P.nfb) +
-                            2 * B_EMFT;
-            for (int g = t; g < 3 * L; g += ROW_THREADS) {
-                const int k = g / 3, f = g - 3 * k;
-                const double2 a = buf[SW(f * FS + k)], b = peer[SW(f * FS + k)];
-                *reinterpret_cast<double2*>(obase + k * mstride + f * 2) = h ? csub(b, a) : cadd(a, b);
-            }
-        }
-        cluster.sync();   // the partner has read this CTA's EMF spectra
-        // M2: (curl B)_theta, (curl B)_phi -> the Lorentz force (:512-519, 635-641, 712-718)
-        {
-            const int fo[2] = {A_CBT, A_CBP};
-            const bool dp[2] = {false, false};
-            row_c2r<N, 2, ZPT>(P, rowbase, h, fo, dp, sm, t, y);
-            const double csc = rowc[RC_CSC], rad = rowc[RC_RAD], rho = rowc[RC_RHO];
-            const double lc = P.lorentz, r2lc = rad * rad * lc, lcr = lc / rho;
-#pragma unroll
-            for (int q = 0; q < ZPT; ++q) {
-                if (!live(q)) continue;
-                const double2 cbt = make_double2(y[0][q].x * csc * orad, y[0][q].y * csc * orad);
-                const double2 cbp = make_double2(y[1][q].x * csc * orad, y[1][q].y * csc * orad);
-                double2& w = acc_at(0, q);
-                double2& pp = acc_at(1, q);
-                double2& z = acc_at(3, q);
-                w.x += r2lc * (cbt.x * bp[q].x - cbp.x * bt[q].x);
-                w.y += r2lc * (cbt.y * bp[q].y - cbp.y * bt[q].y);
-                pp.x -= lcr * (cbp.x * br[q].x - cbr[q].x * bp[q].x);
-                pp.y -= lcr * (cbp.y * br[q].y - cbr[q].y * bp[q].y);
-                z.x -= lcr * (cbr[q].x * bt[q].x - cbt.x * br[q].x);
-                z.y -= lcr * (cbr[q].y * bt[q].y - cbt.y * br[q].y);
-                if constexpr (HEAT) {   // the (curl B)_theta and (curl B)_phi parts
-                    const double oh = rowc[RC_OH];
-                    acc_at(2, q).x += (cbt.x * cbt.x + cbp.x * cbp.x) * oh;
-                    acc_at(2, q).y += (cbt.y * cbt.y + cbp.y * cbp.y) * oh;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    // r2c of W, P, T, Z in place on the accumulators: Z = FFT(y[2n] + i y[2n+1]), then
-    // X_k = e - i conj(w^k) d with e, d the half sums/differences of Z_k, conj Z_{N-k},
-    // one (k, N-k) pair per work item, in place
-    fft_dit<N, 4, ROW_THREADS>(acc, P.twp, t);
-    {
-        const double hsf_pz = rowc[RC_HSF];   // P and Z (f = 1, 3) take the row factor
-        r2c_finish<N>(acc, 4, P.L, P.wr, t, [&](int f) { return (f & 1) ? hsf_pz : 0.5; });
-    }
-    // equatorial fold of PtS_4d_dgpv3 (Legendre_Transforms.F90:1109-1122) with the
-    // partner row: f_even = X(theta) + X(pi - theta) (written by rank 0),
-    // f_odd = X(theta) - X(pi - theta) (written by rank 1)
-    cluster.sync();
-    {
-        const double2* mine = acc;
-        const double2* peer = cluster.map_shared_rank(acc, h ^ 1);
-        const int L = P.L;
-        const long mstride = 2L * (P.nth / 2) * P.ncolb;   // p2b[m][par][theta_h][r][field][2]
-        double* obase = P.p2b + (long)h * (P.nth / 2) * P.ncolb + (long)thh * P.ncolb + (long)r * (2 * P.nfb);
-        for (int g = t; g < 4 * L; g += ROW_THREADS) {   // g = (k, f), f fastest: 64 contiguous bytes per k
-            const int k = g >> 2, f = g & 3;
-            const double2 a = mine[SW(f * FS + k)], b = peer[SW(f * FS + k)];
-            const double2 v = h ? csub(b, a) : cadd(a, b);
-            *reinterpret_cast<double2*>(obase + k * mstride + f * 2) = v;
-        }
-    }
-    // CFL max over the row
-    for (int o = 16; o > 0; o >>= 1) cmax = fmax(cmax, __shfl_down_sync(0xffffffffu, cmax, o));
-    if ((t & 31) == 0) red[t >> 5] = cmax;
-    cluster.sync();   // the partner has finished reading this CTA's spectra
-    if (t == 0) {
-        double v = red[0];
-        for (int i = 1; i < ROW_THREADS / 32; ++i) v = fmax(v, red[i]);
-        atomicMax(P.cfl, (unsigned long long)__double_as_longlong(v));
-    }
-}
-
 FFTPlan make_plan(int n) {
     FFTPlan p{};
     p.n = n;
@@ -975,15 +450,16 @@ void physics_prepare(Ctx& c) {
         RA_CUDA(cudaMalloc(&c.d_twp, std::max<size_t>(tw.size(), 2) * sizeof(double)));
         RA_CUDA(cudaMemcpy(c.d_twp, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
+    physics_pair_prepare(c);
     c.physics3_ok = p3_supported(c.d.nth);
-    // default: all passes in shared memory where that kernel exists (20.7 against 21.5 ms at
-    // n_theta = 768, N_r = 192); the autotuner measures both
-    c.physics_form = physics_form1_supported(c.d.nth) ? 1 : 0;
-    if (!c.physics3_ok && !physics_form1_supported(c.d.nth))
+    // default: the row-pair kernel where it exists (l_max = 511, N_r = 96 with B: 12.6 ms against
+    // 16.6 ms of one CTA per row); the autotuner measures the others too
+    c.physics_form = physics_pair_supported(c.d.nth) ? 1 : 0;
+    if (!c.physics3_ok && !physics_pair_supported(c.d.nth))
         throw ArgError("n_theta " + std::to_string(c.d.nth) + " has no physical-space kernel instance");
-    if (c.mag && !physics_form1_supported(c.d.nth))   // the magnetic terms live in that kernel only
+    if (c.mag && !physics_pair_supported(c.d.nth))   // the magnetic terms live in that kernel only
         throw ArgError("magnetism needs n_theta in 24..768 (2^a or 3*2^a); got " + std::to_string(c.d.nth));
-    if (c.rad.heating && !physics_form1_supported(c.d.nth))   // and so do the heating terms
+    if (c.rad.heating && !physics_pair_supported(c.d.nth))   // and so do the heating terms
         throw ArgError("viscous / ohmic heating needs n_theta in 24..768 (2^a or 3*2^a); got " +
                        std::to_string(c.d.nth));
 }
@@ -992,15 +468,14 @@ void physics_prepare(Ctx& c) {
 // Physical-space kernel with the last FFT pass in registers (N = n_theta with
 // a final radix-3 pass: 384, 768, 1536; N/3 threads per row).
 //
-// The c2r runs the in-place passes of physics_kernel except the last one; the
+// The c2r runs the in-place passes (fft_dif) except the last one; the
 // last (radix-3, stride-1) pass is done in registers by thread t on the three
 // points 3t, 3t+1, 3t+2 of every field, the same points in every batch, so
 // the nonlinear terms are formed where the transform leaves them, and the
 // r2c's first (radix-3) pass is done on the same registers.  Per field this
 // saves the last pass's write and the read-back of the physical values in the
 // c2r, and the first pass's read in the r2c; the velocity stays in registers
-// (nine complex values per thread).  Shared layout and butterfly dealing are
-// physics_kernel's.
+// (nine complex values per thread).
 // ---------------------------------------------------------------------------
 template <int N>
 struct P3 {
@@ -1289,16 +764,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P3<N>::NT, MINB) phy
 // the register-last-pass kernel serves the n_theta whose plan ends in radix 3
 static bool p3_supported(int n) { return n == 384 || n == 768 || n == 1536; }
 
-// n_theta with an instance of physics_kernel (all passes in shared memory)
-bool physics_form1_supported(int n) {
-    switch (n) {
-        case 24: case 32: case 48: case 64: case 96: case 128: case 192: case 256: case 384: case 512: case 768:
-            return true;
-        default:
-            return false;
-    }
-}
-
 void launch_physics(Ctx& c) {
     PhysParams P{};
     P.p2a = c.d_p2a;
@@ -1348,42 +813,7 @@ void launch_physics(Ctx& c) {
         ++c.launches;
         return;
     }
-    auto go = [&](auto kern, int n, size_t smem_units) {
-        const size_t smem = smem_units * sizeof(double2);
-        RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P);
-        (void)n;
-    };
-#define RA_PHYS_CASE(NN)                                                   \
-    case NN:                                                               \
-        if (c.mag && heat)                                                 \
-            go(physics_kernel<NN, true, true>, NN, RowSmem<NN>::SIZE);     \
-        else if (c.mag)                                                    \
-            go(physics_kernel<NN, true, false>, NN, RowSmem<NN>::SIZE);    \
-        else if (heat)                                                     \
-            go(physics_kernel<NN, false, true>, NN, RowSmem<NN>::SIZE);    \
-        else                                                               \
-            go(physics_kernel<NN, false, false>, NN, RowSmem<NN>::SIZE);   \
-        break;
-    const bool heat = c.rad.heating;
-    switch (c.d.nth) {
-        RA_PHYS_CASE(24)
-        RA_PHYS_CASE(32)
-        RA_PHYS_CASE(48)
-        RA_PHYS_CASE(64)
-        RA_PHYS_CASE(96)
-        RA_PHYS_CASE(128)
-        RA_PHYS_CASE(192)
-        RA_PHYS_CASE(256)
-        RA_PHYS_CASE(384)
-        RA_PHYS_CASE(512)
-        RA_PHYS_CASE(768)
-#undef RA_PHYS_CASE
-        default: throw ArgError("n_theta " + std::to_string(c.d.nth) +
-                                " has no physical-space kernel instance (24..768 of the form 2^a or 3*2^a)");
-    }
-    RA_CUDA(cudaGetLastError());
-    ++c.launches;
+    launch_physics_pair(c, P);
 }
 
 __global__ void fft_rows_kernel(double* x, long howmany, const double2* wrg, FFTPlan plan, int inverse) {
@@ -1884,7 +1314,7 @@ void launch_azimuthal_average(Ctx& c, const SliceSpec& S, double* rows) {
 // Shell spectra (Shell_Spectra output; Parallel_IO.F90 Spectral_Prep
 // :973-1047): the quantity on the phi grid (as shell_slice_kernel), its
 // unnormalised r2c (FFT_To_Spectral) and the equatorial fold of PtS with the
-// partner row (theta, pi - theta in one cluster, as physics_kernel), written
+// partner row (theta, pi - theta in one cluster), written
 // into the p2b layout at the column slot slot0 + level index; the forward
 // Legendre transform of that buffer then gives the (l, m) coefficients.
 template <int N>

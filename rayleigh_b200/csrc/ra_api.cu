@@ -916,7 +916,7 @@ static void release(Ctx& c) {
     if (c.d_adapt) cudaFree(c.d_adapt);
     if (c.d_adapt_dt) cudaFree(c.d_adapt_dt);
     lu_workspace_free(c.lu_work);
-    double* bufs[] = {c.d_Ptab, c.d_iPtab, c.d_D, c.d_Dpar, c.d_Dfd, c.d_coef, c.d_radial, c.d_costh, c.d_twid, c.d_twp,
+    double* bufs[] = {c.d_Ptab, c.d_iPtab, c.d_D, c.d_Dpar, c.d_Dfd, c.d_coef, c.d_radial, c.d_costh, c.d_twid, c.d_twp, c.d_twq,
                       c.d_Awpt, c.d_Az,
                       c.d_Ainv_wpt, c.d_Ainv_z,
                       c.d_sol_wpt, c.d_sol_z, c.d_rhs_wpt, c.d_rhs_z, c.d_ab, c.d_g, c.d_s2a, c.d_s2a11,
@@ -1265,7 +1265,7 @@ static std::vector<int> knob_candidates(const Ctx& c, int knob) {
             v.push_back(0);
             v.push_back(2);
         }
-        if (physics_form1_supported(c.d.nth)) v.push_back(1);
+        if (physics_pair_supported(c.d.nth)) v.push_back(1);
         return v;
     }
     std::vector<int> v;   // solve_nc
@@ -1753,7 +1753,7 @@ int ra_set_reference(ra_ctx* ctx, const double* density, const double* dlnrho, c
             if (ohmic_heating_coeff) R.ohm_heat[i] = ohmic_heating_coeff[i];
             heat = heat || R.visc_heat[i] != 0.0 || R.ohm_heat[i] != 0.0;
         }
-        if (heat && !physics_form1_supported(c.d.nth))
+        if (heat && !physics_pair_supported(c.d.nth))
             throw ArgError("viscous / ohmic heating needs n_theta in 24..768 (2^a or 3*2^a)");
         R.heating = heat;
         if (heat || c.mag) c.physics_form = 1;   // the form with the heating and magnetic terms

@@ -176,8 +176,9 @@ struct Ctx {
     double *d_costh = nullptr;                        // [nth] cos, then sin, csc, cot
     double *d_twid = nullptr;                         // [nth] complex exp(2 pi i k / nphi)
     double *d_twp = nullptr;                          // per-pass twiddles of the in-place phi FFT
+    double *d_twq = nullptr;                          // mid-pass twiddles of the row-pair phi FFT
     bool physics3_ok = false;                         // n_theta has a physical-space kernel with the last pass in registers
-    int physics_form = 0;                             // 0/2: that kernel (2 / 1 CTAs per SM), 1: all passes in shared memory
+    int physics_form = 0;                             // 0/2: that kernel (2 / 1 CTAs per SM), 1: the row-pair kernel
     double *d_Awpt = nullptr, *d_Az = nullptr;        // LU factors in block-substitution form [L][3nr][3nr], [L][nr][nr]
     int *d_perm_wpt = nullptr, *d_perm_z = nullptr;   // row permutations of the factors [L][3nr], [L][nr]
     int *d_skip_z = nullptr;                          // [L]: 1 where Z is not solved for (l = 0)
@@ -293,7 +294,10 @@ struct ProbeSet {
 void launch_point_probes(Ctx& c, const SliceSpec& S, const ProbeSet& Q, double* out);
 // tables the launches read, built at set-up (never inside a graph capture)
 void physics_prepare(Ctx& c);
-bool physics_form1_supported(int n_theta);
+struct PhysParams;
+bool physics_pair_supported(int n_theta);
+void physics_pair_prepare(Ctx& c);
+void launch_physics_pair(Ctx& c, PhysParams P);
 void lt_forward_prepare(Ctx& c);
 void solve_prepare(Ctx& c);
 void launch_rlm_b(Ctx& c, double new_ab);
