@@ -21,10 +21,10 @@
 //                       part).  Then y_i = L_ii^-1 (Pb)_i + sum_{j<i} M_ij y_j
 //                       and x_i = U_ii^-1 y_i + sum_{j>i} M_ij x_j are plain
 //                       products, and the substitution runs on the tensor cores.
-//   lu_solve_kernel     DGETRS: one CTA per (system, l, NC right-hand-side
+//   lu_substitute_kernel  DGETRS: one CTA per (system, l, NC right-hand-side
 //                       columns); the permuted columns stay in shared memory
-//                       for both sweeps, the rows of M stream through a
-//                       3-stage cp.async ring, and every block product is an
+//                       for both sweeps, the rows of M stream into fragment
+//                       registers, and every block product is an
 //                       FP64 tensor-core product (mma.sync.m8n8k4.f64).
 //   lu_refine_kernel    FP32 block substitution (the same M rounded to FP32)
 //                       with FP64 residuals b - A x, iterated until the update
@@ -334,25 +334,29 @@ __global__ void __launch_bounds__(256) lu_offdiag_kernel(double* __restrict__ ma
 // columns (P b) sit in shared memory for both sweeps.  For block row i the
 // product over its K range is split between two warp groups (K chunks of 16
 // dealt alternately); warp w owns rows 16 (w mod 4) .. +16 of the block row and
-// all NC columns (2 x NC/8 tensor-core tiles, 2 NC/8 x 2 mma per k-step), and
-// streams ITS OWN rows of M through a private 3-stage cp.async ring, so no
-// CTA-wide barrier is needed until the block row ends: the second group then
-// hands its partial sums to the first through shared memory, which writes the
-// block row's result over its right-hand side.
+// all NC columns (2 x NC/8 tensor-core tiles, 2 NC/8 x 2 mma per k-step).  Each
+// element of M is used by one warp only, so that the warp streams ITS OWN rows
+// straight into fragment registers, two chunks ahead (a lane takes two
+// neighbouring k of a row with one 16-byte load; the k of an 8-wide group are
+// dealt to two k-steps accordingly), and no CTA-wide barrier is needed until the
+// block row ends: the second group then hands its partial sums to the first
+// through shared memory, which writes the block row's result over its
+// right-hand side.
+// What bounds it: on small systems the chain of one CTA (load the columns, 2 nblk
+// dependent block rows, store), on large ones the FP64 tensor rate.  Hence the
+// columns arrive by 8-byte cp.async, all in flight together (one load a column
+// after the other took longer than the substitution below n ~ 200), and every
+// system of the step goes out as one launch where two CTAs fit an SM (n <= 384).
+// Without a shared-memory ring for M the block takes 65 KB at n = 144 (three CTAs
+// per SM instead of one) and 98 KB at n = 288 (two).
 constexpr int LS_KC = 16;                 // K per chunk
-constexpr int LS_RS = LS_KC + 4;          // ring row stride (doubles): conflict-free A fragments
-constexpr int LS_STAGES = 3;
 constexpr int LS_WARPS = 8, LS_THREADS = 32 * LS_WARPS;
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int src_bytes) {
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(src_bytes));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -361,43 +365,36 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 }
 
 // The column block in shared memory, [row][NC] with the columns of row i
-// permuted by XOR with h(i) = 8 (i mod 2) + (i/2 mod 8): over a warp, a B
-// fragment (rows k..k+3, k = 0 mod 4, 8 columns) and a walk down 32
+// permuted by XOR with h(i) = 8 i_1 + (i_0 + 2 i_2 + 4 i_3) (bits of i): a B
+// fragment (rows k + 2 tig, k = 0 mod 8, 8 columns) and a walk down 32
 // consecutive rows of one column both touch every 8-byte bank exactly twice.
-// (A layout that is also conflict-free per half warp, h(i) = 4 (i mod 4) +
-// (i/4 mod 4), measured 35 % slower: 0.92 against 0.68 ms at l_max = 127,
-// N_r = 192, with a third of the shared wavefronts.)
 template <int NC>
 __device__ __forceinline__ int xs_index(int i, int c) {
-    return i * NC + (c ^ (((i & 1) << 3) | ((i >> 1) & 7)));
-}
-
-// chunk j of block row ib (both sweeps): K start
-__device__ __forceinline__ int chunk_k0(bool backward, int ib, int j) {
-    return backward ? ib * SB + j * LS_KC : j * LS_KC;
+    return i * NC + (c ^ (((i & 2) << 2) | (i & 1) | ((i >> 1) & 6)));
 }
 
 template <int NC>
 struct LuSolveShape {
     static size_t smem(int n) {
         const int nrow = (n + SB - 1) / SB * SB;
-        return ((size_t)nrow * NC + (size_t)LS_WARPS * LS_STAGES * 16 * LS_RS + (size_t)SB * NC) * sizeof(double);
+        return ((size_t)nrow * NC + (size_t)SB * NC) * sizeof(double) + (size_t)nrow * sizeof(int);
     }
 };
 
 template <int NC>
-__global__ void __launch_bounds__(LS_THREADS) lu_solve_kernel(const int4* __restrict__ tiles, LuSys S, int mode,
-                                                              int ncols_fixed) {
+__global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4* __restrict__ tiles, LuSysSet set,
+                                                                      int mode, int ncols_fixed) {
     constexpr int NT = NC / 8;               // n-tiles per warp
     extern __shared__ __align__(16) double ssm[];
     const int4 tl = tiles[blockIdx.x];
+    const LuSys S = set.s[tl.x];
     const int l = tl.y, c0 = tl.z * NC, n = S.n;
     const int nblk = (n + SB - 1) / SB, nrow = nblk * SB;
     double* Xs = ssm;                                      // [nrow][NC]
-    double* ring_all = Xs + (size_t)nrow * NC;             // [warp][stage][16][LS_RS]
-    double* red = ring_all + LS_WARPS * LS_STAGES * 16 * LS_RS;   // [SB][NC] second group's partial sums
-    const double* M = S.M + (size_t)l * n * n;
-    const int* perm = S.perm + (size_t)l * n;
+    double* red = Xs + (size_t)nrow * NC;                  // [SB][NC] second group's partial sums
+    int* inv = reinterpret_cast<int*>(red + SB * NC);      // [n] the row a right-hand-side entry goes to
+    const double* __restrict__ M = S.M + (size_t)l * n * n;
+    const int* __restrict__ perm = S.perm + (size_t)l * n;
     const double* rhs = nullptr;
     double* sol;
     int ncol;
@@ -415,38 +412,27 @@ __global__ void __launch_bounds__(LS_THREADS) lu_solve_kernel(const int4* __rest
         ncol = ncols_fixed;
     }
     const int t = threadIdx.x;
-    // permuted right-hand sides (P b), zero past n and past the last column; threads walk rows
-    for (int c = 0; c < NC; ++c) {
-        const int col = c0 + c;
-        for (int i = t; i < nrow; i += LS_THREADS) {
-            double v = 0.0;
-            if (i < n && col < ncol)
-                v = (mode == LU_MODE_INVERSE) ? (perm[i] == col ? 1.0 : 0.0) : rhs[(size_t)col * n + perm[i]];
-            Xs[xs_index<NC>(i, c)] = v;
-        }
-    }
     const int lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
     const int rgp = warp & 3, grp = warp >> 2;             // row group (16 rows), K group
-    double* ring = ring_all + warp * LS_STAGES * 16 * LS_RS;
-    // this warp's chunks in order over both sweeps: (block row q-th, chunk j = grp, grp + 2, ...)
-    // forward block ib has 4 (ib + 1) chunks; backward block ib has 4 (nblk - ib)
+    // this warp's chunks in order over both sweeps: (block row q-th, chunk j = grp, grp + 2, ...);
+    // forward block ib has 4 (ib + 1) chunks from k = 0 on; backward block ib has 4 (nblk - ib) from
+    // its own first row on
     auto nchunks = [&](bool bw, int ib) { return bw ? 4 * (nblk - ib) : 4 * (ib + 1); };
-    // issue the copy of the warp's chunk number s (its 16 rows x 16 k of M)
     int f_bw = 0, f_q = 0, f_j = grp;                      // fetch cursor: sweep, block row ordinal, chunk
-    auto fetch_next = [&](int stage) {
+    auto fetch = [&](double2 (&a)[2][2]) {                 // rows g, g + 8 of the warp's 16; k = 8 h + 2 tig + {0, 1}
         if (f_bw < 2) {
             const bool bw = f_bw == 1;
             const int ib = bw ? nblk - 1 - f_q : f_q;
-            const int k0 = chunk_k0(bw, ib, f_j);
-            double* dst = ring + stage * 16 * LS_RS;
+            const int gk0 = (bw ? ib * SB : 0) + f_j * LS_KC + 2 * tig;
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {           // 16 rows x 8 pieces of 16 bytes = 128 pieces, 4 per lane
-                const int e = lane + 32 * p, r = e >> 3, pc = e & 7;
-                const int gr = ib * SB + rgp * 16 + r, gk = k0 + 2 * pc;
-                const bool ok = gr < n && gk < n;
-                cp_async16(dst + r * LS_RS + 2 * pc, ok ? (const void*)(M + (size_t)gr * n + gk) : (const void*)M,
-                           ok ? 16 : 0);
+            for (int mi = 0; mi < 2; ++mi) {
+                const int gr = ib * SB + rgp * 16 + mi * 8 + g;
+                const double* row = M + (size_t)gr * n;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    a[mi][h] = (gr < n && gk0 + 8 * h < n) ? __ldg(reinterpret_cast<const double2*>(row + gk0 + 8 * h))
+                                                           : make_double2(0.0, 0.0);
             }
             f_j += 2;
             if (f_j >= nchunks(bw, ib)) {
@@ -457,51 +443,79 @@ __global__ void __launch_bounds__(LS_THREADS) lu_solve_kernel(const int4* __rest
                 }
             }
         }
-        cp_async_commit();
     };
+    double2 a0[2][2] = {}, a1[2][2] = {};
+    fetch(a0);
+    fetch(a1);
+    // permuted right-hand sides (P b), zero past n and past the last column; the entries of a column are
+    // read in order and go to their rows
+    if (mode == LU_MODE_INVERSE) {
+        for (int i = t; i < nrow; i += LS_THREADS)
+#pragma unroll 4
+            for (int c = 0; c < NC; ++c) Xs[xs_index<NC>(i, c)] = (i < n && perm[i] == c0 + c) ? 1.0 : 0.0;
+    } else {
+        for (int i = t; i < n; i += LS_THREADS) inv[perm[i]] = i;
+        for (int i = n + t; i < nrow; i += LS_THREADS)
+            for (int c = 0; c < NC; ++c) Xs[xs_index<NC>(i, c)] = 0.0;
+        __syncthreads();
+        for (int i = t; i < n; i += LS_THREADS) {
+            const int row = inv[i];
+            const double* src = rhs + (size_t)c0 * n + i;
+#pragma unroll 8
+            for (int c = 0; c < NC; ++c) {
+                if (c0 + c < ncol)
+                    cp_async8(Xs + xs_index<NC>(row, c), src + (size_t)c * n);
+                else
+                    Xs[xs_index<NC>(row, c)] = 0.0;
+            }
+        }
+        cp_async_wait_all();
+    }
     __syncthreads();   // Xs complete
-#pragma unroll
-    for (int st = 0; st < LS_STAGES - 1; ++st) fetch_next(st);
-    int stage = 0;
     for (int bwi = 0; bwi < 2; ++bwi) {
         const bool bw = bwi == 1;
         for (int q = 0; q < nblk; ++q) {
             const int ib = bw ? nblk - 1 - q : q;
-            const int nch = nchunks(bw, ib);
+            const int nch = nchunks(bw, ib), kb = bw ? ib * SB : 0;
             double acc[2][NT][2];
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
                 for (int ni = 0; ni < NT; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
-            for (int j = grp; j < nch; j += 2) {
-                cp_async_wait<LS_STAGES - 2>();
-                __syncwarp();
-                fetch_next((stage + LS_STAGES - 1) % LS_STAGES);
-                const double* a_st = ring + stage * 16 * LS_RS;
-                const int k0 = chunk_k0(bw, ib, j);
-                const bool diag = k0 >= ib * SB && k0 < ib * SB + SB;
-#pragma unroll
-                for (int kk = 0; kk < LS_KC; kk += 4) {
-                    const int kg = k0 + kk + tig;
-                    double a[2], b[NT];
-#pragma unroll
-                    for (int mi = 0; mi < 2; ++mi) {
-                        const int r = mi * 8 + g;
-                        double v = a_st[r * LS_RS + kk + tig];
-                        if (diag) {
-                            const int rg = ib * SB + rgp * 16 + r;
-                            v = bw ? (kg >= rg ? v : 0.0) : (kg < rg ? v : (kg == rg ? 1.0 : 0.0));
-                        }
-                        a[mi] = v;
-                    }
-#pragma unroll
-                    for (int ni = 0; ni < NT; ++ni) b[ni] = Xs[xs_index<NC>(kg, ni * 8 + g)];
+            auto multiply = [&](double2 (&a)[2][2], int j) {
+                const int k0 = kb + j * LS_KC;
+                if (k0 >= ib * SB && k0 < ib * SB + SB) {   // the diagonal block: L^-1 (unit) or U^-1
 #pragma unroll
                     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-                        for (int ni = 0; ni < NT; ++ni) dmma884(acc[mi][ni], a[mi], b[ni]);
+                        for (int h = 0; h < 2; ++h) {
+                            const int rg = ib * SB + rgp * 16 + mi * 8 + g, kg = k0 + 8 * h + 2 * tig;
+                            double2& v = a[mi][h];
+                            v.x = bw ? (kg >= rg ? v.x : 0.0) : (kg < rg ? v.x : (kg == rg ? 1.0 : 0.0));
+                            v.y = bw ? (kg + 1 >= rg ? v.y : 0.0) : (kg + 1 < rg ? v.y : (kg + 1 == rg ? 1.0 : 0.0));
+                        }
                 }
-                stage = (stage + 1) % LS_STAGES;
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const int kg = k0 + 8 * h + 2 * tig + s;
+                        double b[NT];
+#pragma unroll
+                        for (int ni = 0; ni < NT; ++ni) b[ni] = Xs[xs_index<NC>(kg, ni * 8 + g)];
+#pragma unroll
+                        for (int mi = 0; mi < 2; ++mi) {
+                            const double av = s ? a[mi][h].y : a[mi][h].x;
+#pragma unroll
+                            for (int ni = 0; ni < NT; ++ni) dmma884(acc[mi][ni], av, b[ni]);
+                        }
+                    }
+            };
+            for (int j = grp; j < nch; j += 4) {   // an even number of chunks per group
+                multiply(a0, j);
+                fetch(a0);
+                multiply(a1, j + 2);
+                fetch(a1);
             }
             // the second K group hands over its partial sums; the first writes the block row
             if (grp == 1) {
@@ -528,9 +542,10 @@ __global__ void __launch_bounds__(LS_THREADS) lu_solve_kernel(const int4* __rest
             __syncthreads();
         }
     }
-    cp_async_wait<0>();
-    for (int c = 0; c < NC && c0 + c < ncol; ++c)
-        for (int i = t; i < n; i += LS_THREADS) sol[(size_t)(c0 + c) * n + i] = Xs[xs_index<NC>(i, c)];
+    for (int i = t; i < n; i += LS_THREADS)
+#pragma unroll 8
+        for (int c = 0; c < NC; ++c)
+            if (c0 + c < ncol) sol[(size_t)(c0 + c) * n + i] = Xs[xs_index<NC>(i, c)];
 }
 
 // ---------------------------------------------------------------------------
@@ -656,9 +671,9 @@ static void set_smem(F* kern, size_t bytes) {
     RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
-int lu_nc_for(int n) {
-    return LuSolveShape<32>::smem(n) <= (size_t)(227 << 10) ? 32 : 16;
-}
+// 32 columns a CTA up to n = 576, 16 above (their blocks fill the same shared memory at twice the n)
+int lu_nc_for(int n) { return n <= 576 ? 32 : 16; }
+constexpr int LS_MAX_N = 1216;
 
 void lu_workspace(LuWork& w, int n, int count) {
     const int nblk = (n + SB - 1) / SB;
@@ -709,21 +724,20 @@ int lu_factor_batch(cudaStream_t st, LuWork& w, double* d_mats, int* d_perm, int
     return 0;
 }
 
-void launch_lu_solve(cudaStream_t st, const int* d_tiles, int ntiles, const LuSys& sys, int mode, int ncols_fixed,
+void launch_lu_solve(cudaStream_t st, const int* d_tiles, int ntiles, const LuSysSet& set, int mode, int ncols_fixed,
                      int nc) {
     if (ntiles == 0) return;
-    if (nc == 32) {
-        const size_t sm = LuSolveShape<32>::smem(sys.n);
-        set_smem(lu_solve_kernel<32>, sm);
-        lu_solve_kernel<32><<<ntiles, LS_THREADS, sm, st>>>(reinterpret_cast<const int4*>(d_tiles), sys, mode,
-                                                            ncols_fixed);
-    } else {
-        const size_t sm = LuSolveShape<16>::smem(sys.n);
-        if (sm > (size_t)(227 << 10)) throw ArgError("per-l matrix order too large for the block substitution");
-        set_smem(lu_solve_kernel<16>, sm);
-        lu_solve_kernel<16><<<ntiles, LS_THREADS, sm, st>>>(reinterpret_cast<const int4*>(d_tiles), sys, mode,
-                                                            ncols_fixed);
-    }
+    int n = 0;
+    for (int i = 0; i < set.count; ++i) n = std::max(n, set.s[i].n);
+    if (n > LS_MAX_N) throw ArgError("per-l matrix order too large for the block substitution");
+    auto go = [&](auto kern, size_t sm) {
+        set_smem(kern, sm);
+        kern<<<ntiles, LS_THREADS, sm, st>>>(reinterpret_cast<const int4*>(d_tiles), set, mode, ncols_fixed);
+    };
+    if (nc == 32)
+        go(lu_substitute_kernel<32>, LuSolveShape<32>::smem(n));
+    else
+        go(lu_substitute_kernel<16>, LuSolveShape<16>::smem(n));
     RA_CUDA(cudaGetLastError());
 }
 
@@ -768,7 +782,7 @@ static T* upload_vec(Ctx& c, const std::vector<T>& v) {
     return d;
 }
 
-// Tile lists of the step's substitution (one launch per system) and, in the
+// Tile lists of the step's substitution (W-P-T, then Z, then C and A) and, in the
 // mixed form, of the explicit inverses; built once at set-up, since no
 // allocation may run while a step is captured.
 void solve_prepare(Ctx& c) {
@@ -787,10 +801,15 @@ void rebuild_solve_tiles(Ctx& c) {
         cnt = (int)(t.size() / 4);
         d = upload_vec(c, t);
     };
-    std::vector<int> step_cols(L);
-    for (int l = 0; l < L; ++l) step_cols[l] = 2 * (l + 1);
-    make(c.d_solve_tiles, c.n_solve_tiles, step_cols, c.solve_nc);
-    make(c.d_solve_tiles_z, c.n_solve_tiles_z, step_cols, c.solve_nc_z);
+    if (!c.d_solve_tiles) {
+        std::vector<int> cols(L), t;
+        for (int l = 0; l < L; ++l) cols[l] = 2 * (l + 1);
+        lu_append_tiles(t, 0, L, cols, c.solve_nc);
+        c.n_solve_tiles = (int)(t.size() / 4);
+        for (int sys = 1; sys < (c.mag ? 4 : 2); ++sys) lu_append_tiles(t, sys, L, cols, c.solve_nc_z);
+        c.n_solve_tiles_z = ((int)(t.size() / 4) - c.n_solve_tiles) / (c.mag ? 3 : 1);
+        c.d_solve_tiles = upload_vec(c, t);
+    }
     if (c.mixed_solve) {
         make(c.d_inv_sol_tiles, c.n_inv_sol_tiles, std::vector<int>(L, 3 * nr), c.solve_nc);
         make(c.d_inv_sol_tiles_z, c.n_inv_sol_tiles_z, std::vector<int>(L, nr), c.solve_nc_z);
@@ -815,14 +834,14 @@ void factor_matrices(Ctx& c) {
         if (bad) throw SingularError("singular A matrix at l = " + std::to_string(bad - 1));
     }
     if (c.mixed_solve) {
-        const LuSys s0{c.d_Awpt, c.d_perm_wpt, nullptr, c.d_Ainv_wpt, 3 * nr};
-        const LuSys s1{c.d_Az, c.d_perm_z, nullptr, c.d_Ainv_z, nr};
+        const LuSysSet s0{{{c.d_Awpt, c.d_perm_wpt, nullptr, c.d_Ainv_wpt, 3 * nr}}, 1};
+        const LuSysSet s1{{{c.d_Az, c.d_perm_z, nullptr, c.d_Ainv_z, nr}}, 1};
         launch_lu_solve(c.stream, c.d_inv_sol_tiles, c.n_inv_sol_tiles, s0, LU_MODE_INVERSE, 0, c.solve_nc);
         launch_lu_solve(c.stream, c.d_inv_sol_tiles_z, c.n_inv_sol_tiles_z, s1, LU_MODE_INVERSE, 0, c.solve_nc_z);
         c.launches += 2;
         if (c.mag) {   // the C and A systems go through the split products too
-            const LuSys sc{c.d_Ac, c.d_perm_c, nullptr, c.d_Ainv_c, nr};
-            const LuSys sa{c.d_Aa, c.d_perm_a, nullptr, c.d_Ainv_a, nr};
+            const LuSysSet sc{{{c.d_Ac, c.d_perm_c, nullptr, c.d_Ainv_c, nr}}, 1};
+            const LuSysSet sa{{{c.d_Aa, c.d_perm_a, nullptr, c.d_Ainv_a, nr}}, 1};
             launch_lu_solve(c.stream, c.d_inv_sol_tiles_z, c.n_inv_sol_tiles_z, sc, LU_MODE_INVERSE, 0, c.solve_nc_z);
             launch_lu_solve(c.stream, c.d_inv_sol_tiles_z, c.n_inv_sol_tiles_z, sa, LU_MODE_INVERSE, 0, c.solve_nc_z);
             c.launches += 2;
@@ -831,27 +850,29 @@ void factor_matrices(Ctx& c) {
     RA_CUDA(cudaStreamSynchronize(c.stream));
 }
 
-// Implicit_Solve (Linear_Solve.F90:423-457): x = A_l^-1 b for every (system, l).
-void launch_solve(Ctx& c) {
+// Implicit_Solve (Linear_Solve.F90:423-457): x = A_l^-1 b for every (system, l): W-P-T and Z, and
+// with magnetic the C and A equations (l = 0 is the identity there).  One launch where its shared
+// memory (set by the W-P-T columns) still lets two CTAs share an SM, n <= 384; above that the small
+// systems go out on their own, three CTAs an SM.
+void launch_solve(Ctx& c, bool magnetic) {
     if (!c.d_solve_tiles) throw ArgError("solve tiles not prepared (solve_prepare runs at set-up)");
-    const int nr = c.d.nr;
-    const LuSys s0{c.d_Awpt, c.d_perm_wpt, c.d_rhs_wpt, c.d_sol_wpt, 3 * nr};
-    const LuSys s1{c.d_Az, c.d_perm_z, c.d_rhs_z, c.d_sol_z, nr};
-    launch_lu_solve(c.stream, c.d_solve_tiles, c.n_solve_tiles, s0, LU_MODE_STEP, 0, c.solve_nc);
-    launch_lu_solve(c.stream, c.d_solve_tiles_z, c.n_solve_tiles_z, s1, LU_MODE_STEP, 0, c.solve_nc_z);
-    c.launches += 2;
-}
-
-// The C and A equations of the magnetic set (both precision forms): FP64 LU substitution
-// with the Z system's tile list (same size, same columns per l; l = 0 is the identity).
-void launch_solve_mag(Ctx& c) {
-    if (!c.d_solve_tiles_z) throw ArgError("solve tiles not prepared (solve_prepare runs at set-up)");
-    const int nr = c.d.nr;
-    const LuSys sc{c.d_Ac, c.d_perm_c, c.d_rhs_c, c.d_sol_c, nr};
-    const LuSys sa{c.d_Aa, c.d_perm_a, c.d_rhs_a, c.d_sol_a, nr};
-    launch_lu_solve(c.stream, c.d_solve_tiles_z, c.n_solve_tiles_z, sc, LU_MODE_STEP, 0, c.solve_nc_z);
-    launch_lu_solve(c.stream, c.d_solve_tiles_z, c.n_solve_tiles_z, sa, LU_MODE_STEP, 0, c.solve_nc_z);
-    c.launches += 2;
+    const int nr = c.d.nr, rest = c.n_solve_tiles_z * (magnetic ? 3 : 1);
+    const LuSysSet set{{{c.d_Awpt, c.d_perm_wpt, c.d_rhs_wpt, c.d_sol_wpt, 3 * nr},
+                        {c.d_Az, c.d_perm_z, c.d_rhs_z, c.d_sol_z, nr},
+                        {c.d_Ac, c.d_perm_c, c.d_rhs_c, c.d_sol_c, nr},
+                        {c.d_Aa, c.d_perm_a, c.d_rhs_a, c.d_sol_a, nr}},
+                       4};
+    if (c.solve_nc == c.solve_nc_z && 3 * nr <= 384) {
+        launch_lu_solve(c.stream, c.d_solve_tiles, c.n_solve_tiles + rest, set, LU_MODE_STEP, 0, c.solve_nc);
+        c.launches += 1;
+    } else {
+        LuSysSet small = set;
+        small.s[0].n = 0;   // no tile names it
+        launch_lu_solve(c.stream, c.d_solve_tiles, c.n_solve_tiles, set, LU_MODE_STEP, 0, c.solve_nc);
+        launch_lu_solve(c.stream, c.d_solve_tiles + 4 * (size_t)c.n_solve_tiles, rest, small, LU_MODE_STEP, 0,
+                        c.solve_nc_z);
+        c.launches += 2;
+    }
 }
 
 }  // namespace ra

@@ -927,7 +927,7 @@ static void release(Ctx& c) {
         if (b) cudaFree(b);
     int* ibufs[] = {c.d_ltiles, c.d_inv_tiles, c.d_fwd_tiles, c.d_cheb_tiles, c.d_solve_tiles, c.d_status,
                     c.d_perm_wpt, c.d_perm_z, c.d_skip_z, c.d_inv_sol_tiles, c.d_inv_sol_tiles_z,
-                    c.d_solve_tiles_z, c.d_perm_c, c.d_perm_a};
+                    c.d_perm_c, c.d_perm_a};
     for (int* b : ibufs)
         if (b) cudaFree(b);
     if (c.d_cfl) cudaFree(c.d_cfl);
@@ -982,8 +982,7 @@ static void run_stage(Ctx& c, int k, double new_ab, double old_ab) {
             if (c.mixed_solve) {
                 launch_solve_mixed(c);   // every system, C and A included
             } else {
-                launch_solve(c);
-                if (c.mag) launch_solve_mag(c);
+                launch_solve(c, c.mag);
             }
             break;
     }
@@ -1335,7 +1334,7 @@ static void autotune(Ctx& c, int nreps, double* ms_out) {
                     launch_physics(c);
                 } else {
                     if (c.mixed_solve) return;   // the mixed form solves by split products
-                    launch_solve(c);
+                    launch_solve(c, false);
                 }
             };
             run();

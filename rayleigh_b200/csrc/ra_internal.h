@@ -104,6 +104,11 @@ struct LuSys {
     double* sol;
     int n;
 };
+// the systems of one launch; a tile names its system
+struct LuSysSet {
+    LuSys s[4];
+    int count;
+};
 // where a tile's right-hand-side columns are: the step's equation-set layout
 // (2 (l+1) columns from l (l+1)/2 on), the identity (explicit inverse), or a
 // fixed number of columns per l ([l][ncols][n])
@@ -186,7 +191,6 @@ struct Ctx {
     int solve_nc = 32, solve_nc_z = 32;               // right-hand-side columns per substitution CTA (W-P-T, Z)
     int n_inv_sol_tiles = 0, n_inv_sol_tiles_z = 0, n_solve_tiles_z = 0;
     int *d_inv_sol_tiles = nullptr, *d_inv_sol_tiles_z = nullptr;   // tile lists of the explicit inverses (mixed form)
-    int* d_solve_tiles_z = nullptr;                   // the Z system's substitution tiles
     int *d_ltiles = nullptr;                          // LT tile lists
     int n_inv_tiles = 0, n_fwd_tiles = 0, n_cheb_tiles = 0, n_solve_tiles = 0;
     int *d_inv_tiles = nullptr, *d_fwd_tiles = nullptr, *d_cheb_tiles = nullptr, *d_solve_tiles = nullptr;
@@ -298,13 +302,14 @@ struct PhysParams;
 bool physics_pair_supported(int n_theta);
 void physics_pair_prepare(Ctx& c);
 void launch_physics_pair(Ctx& c, PhysParams P);
+bool rows_pair_supported(const Ctx& c);
+void launch_rows_pair(Ctx& c, bool to_rows, double* p2, double* rows, int nfr);
 void lt_forward_prepare(Ctx& c);
 void solve_prepare(Ctx& c);
 void launch_rlm_b(Ctx& c, double new_ab);
 void launch_post_assemble_mag(Ctx& c, double old_ab);
 void launch_rlm_b_mag(Ctx& c, double new_ab);
-void launch_solve_mag(Ctx& c);
-void launch_solve(Ctx& c);
+void launch_solve(Ctx& c, bool magnetic);
 void factor_matrices(Ctx& c);
 void rebuild_solve_tiles(Ctx& c);   // LU of the loaded per-l matrices (+ explicit inverses in the mixed form)
 // k_solve.cu
@@ -313,7 +318,7 @@ void lu_workspace(LuWork& w, int n, int count);
 void lu_workspace_free(LuWork& w);
 int lu_factor_batch(cudaStream_t st, LuWork& w, double* d_mats, int* d_perm, int n, int count, const int* d_skip,
                     long* launches);
-void launch_lu_solve(cudaStream_t st, const int* d_tiles, int ntiles, const LuSys& sys, int mode, int ncols_fixed,
+void launch_lu_solve(cudaStream_t st, const int* d_tiles, int ntiles, const LuSysSet& set, int mode, int ncols_fixed,
                      int nc);
 void lu_append_tiles(std::vector<int>& t, int sys, int L, const std::vector<int>& ncols_of_l, int nc);
 void launch_lu_refine(cudaStream_t st, const int* d_tiles, int ntiles, const LuSys& s, const float* d_mf,

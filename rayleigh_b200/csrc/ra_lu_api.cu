@@ -211,7 +211,7 @@ int ra_lu_solve(ra_lu* lu, const double* b, double* x, int ncols, int mode, int*
         RA_CUDA(cudaEventRecord(e0, lu->stream));
         const LuSys s{lu->d_m, lu->d_perm, lu->d_b, lu->d_x, n};
         if (mode == RA_SOLVE_FP64)
-            launch_lu_solve(lu->stream, lu->d_tiles, lu->ntiles, s, LU_MODE_FIXED, ncols, nc);
+            launch_lu_solve(lu->stream, lu->d_tiles, lu->ntiles, LuSysSet{{s}, 1}, LU_MODE_FIXED, ncols, nc);
         else
             launch_lu_refine(lu->stream, lu->d_tiles, lu->ntiles, s, lu->d_mf, lu->d_a, ncols, lu->d_iters);
         RA_CUDA(cudaEventRecord(e1, lu->stream));
