@@ -5,7 +5,9 @@
 // FFTs (FFT_To_Physical / FFT_To_Spectral, Fourier_Transform.F90:100-183) on
 // rows of n_phi + 2 doubles.  The step fuses the last two into its
 // physical-space kernel; this path serves batches of arbitrary fields (the
-// transform sweep) with the operands in device memory.
+// transform sweep) with the operands in device memory, and runs them as one kernel each way on
+// row pairs (k_phi_rows.cu); the relayout kernels below serve n_theta = 1536 and an l_max above
+// n_phi / 3.
 #include <cmath>
 
 #include "ra_internal.h"
@@ -89,6 +91,7 @@ void transform_dev(Ctx& c, int direction, int precision, double* spec, double* g
                    double* stage_ms) {
     const int ncol = 2 * nfr;
     const long rows = (long)c.d.nth * nfr;
+    const bool pair = rows_pair_supported(c);
     cudaEvent_t ev[4];
     for (auto& e : ev) RA_CUDA(cudaEventCreate(&e));
     auto product = [&] {
@@ -109,15 +112,23 @@ void transform_dev(Ctx& c, int direction, int precision, double* spec, double* g
         RA_CUDA(cudaEventRecord(ev[0], c.stream));
         product();
         RA_CUDA(cudaEventRecord(ev[1], c.stream));
-        launch_relayout(c, true, work, grid, nfr);
-        RA_CUDA(cudaEventRecord(ev[2], c.stream));
-        launch_fft_rows(c, grid, rows, 1);
+        if (pair) {   // unfolded and transformed in one pass: no relayout time
+            RA_CUDA(cudaEventRecord(ev[2], c.stream));
+            launch_rows_pair(c, true, work, grid, nfr);
+        } else {
+            launch_relayout(c, true, work, grid, nfr);
+            RA_CUDA(cudaEventRecord(ev[2], c.stream));
+            launch_fft_rows(c, grid, rows, 1);
+        }
         RA_CUDA(cudaEventRecord(ev[3], c.stream));
     } else {                // physical -> spectral: r2c, fold, PtS
         RA_CUDA(cudaEventRecord(ev[0], c.stream));
-        launch_fft_rows(c, grid, rows, 0);
+        if (pair)
+            launch_rows_pair(c, false, work, grid, nfr);
+        else
+            launch_fft_rows(c, grid, rows, 0);
         RA_CUDA(cudaEventRecord(ev[1], c.stream));
-        launch_relayout(c, false, work, grid, nfr);
+        if (!pair) launch_relayout(c, false, work, grid, nfr);
         RA_CUDA(cudaEventRecord(ev[2], c.stream));
         product();
         RA_CUDA(cudaEventRecord(ev[3], c.stream));
