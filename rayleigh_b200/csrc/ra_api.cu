@@ -398,56 +398,115 @@ static void reference_setup(Ctx& c) {
     }
 }
 
+// The per-l systems
+enum { SYS_WPT, SYS_Z, SYS_C, SYS_A };
+
+// The matrices of one l on the host: term (eq, var, d) adds a(i) D_d(i, :) to the rows of eq in the
+// columns of var; a boundary row is cleared and takes amp D_d over the dealiased columns.
+struct MatrixSink {
+    const Ctx& c;
+    std::vector<double> M[4];
+    explicit MatrixSink(const Ctx& ctx) : c(ctx) {}
+    int order(int sys) const { return sys == SYS_WPT ? 3 * c.d.nr : c.d.nr; }
+    void begin() {
+        for (int s = 0; s < 4; ++s) M[s].assign((size_t)order(s) * order(s), 0.0);
+    }
+    void add(int sys, int eq, int var, int d, const std::vector<double>& a) {
+        const int nr = c.d.nr, n = order(sys);
+        const double* Dd = c.cheb_D.data() + (size_t)d * nr * nr;
+        for (int i = 0; i < nr; ++i)
+            for (int j = 0; j < nr; ++j) M[sys][(size_t)(eq * nr + i) * n + var * nr + j] += a[i] * Dd[(size_t)i * nr + j];
+    }
+    void clear(int sys, int row) {
+        const int n = order(sys);
+        std::fill(M[sys].begin() + (size_t)row * n, M[sys].begin() + (size_t)(row + 1) * n, 0.0);
+    }
+    void bc(int sys, int row, int col0, int d, double amp) {
+        const int nr = c.d.nr, n = order(sys);
+        const double* Dd = c.cheb_D.data() + ((size_t)d * nr + row % nr) * nr;
+        for (int j = 0; j < c.d.rda - 1; ++j) M[sys][(size_t)row * n + col0 + j] += amp * Dd[j];
+    }
+};
+
+// The same as the operands of the device assembly: the shape (shared by every l > 0) and the l's
+// profiles and boundary amplitudes.
+struct RecipeSink {
+    AsmShape S{};
+    double *amp, *bamp;
+    int nr;
+    RecipeSink(double* a, double* b, int n) : amp(a), bamp(b), nr(n) {}
+    void add(int sys, int eq, int var, int d, const std::vector<double>& a) {
+        if (S.nterm == AsmShape::MAXT) throw ArgError("too many terms in an implicit matrix");
+        S.sys[S.nterm] = (signed char)sys;
+        S.eq[S.nterm] = (signed char)eq;
+        S.var[S.nterm] = (signed char)var;
+        S.d[S.nterm] = (signed char)d;
+        std::copy(a.begin(), a.end(), amp + (size_t)S.nterm * nr);
+        ++S.nterm;
+    }
+    void clear(int sys, int row) {
+        if (S.nclear == AsmShape::MAXB) throw ArgError("too many boundary rows");
+        S.clear_sys[S.nclear] = (signed char)sys;
+        S.clear_row[S.nclear++] = row;
+    }
+    void bc(int sys, int row, int col0, int d, double a) {
+        if (S.nbc == AsmShape::MAXB) throw ArgError("too many boundary terms");
+        S.bc_sys[S.nbc] = (signed char)sys;
+        S.bc_d[S.nbc] = (signed char)d;
+        S.bc_row[S.nbc] = row;
+        S.bc_col[S.nbc] = col0;
+        bamp[S.nbc++] = a;
+    }
+};
+
 // The C (poloidal) and A (toroidal) systems of one l > 0 (Sphere_Linear_Terms.F90:473-499)
 // with the insulating boundaries (:1041-1077): A = 0 at both; C matched to a potential
 // field, dC/dr + l C / r = 0 at the top and dC/dr - (l + 1) C / r = 0 at the bottom.
 // coefm[NMSLOT][nr]: the Post_Solve coefficients (C,C,0) (C,C,2) (A,A,0) (A,A,1) (A,A,2).
-static void build_l_mag(const Ctx& c, int l, std::vector<double>& Cm, std::vector<double>& Am, double* coefm) {
-    const int nr = c.d.nr, rda = c.d.rda;
+template <class Sink>
+static void terms_l_mag(const Ctx& c, int l, Sink& out, double* coefm) {
+    const int nr = c.d.nr;
     const double dt = c.dt, al = c.cfg.alpha_implicit;
     const double lf = -dt * al, rf = dt * (1.0 - al);
-    const double* D = c.cheb_D.data();
     const std::vector<double>& r = c.rad.radius;
     const std::vector<double>& eta = c.rad.eta;
-    Cm.assign((size_t)nr * nr, 0.0);
-    Am.assign((size_t)nr * nr, 0.0);
     std::fill(coefm, coefm + (size_t)NMSLOT * nr, 0.0);
     if (l == 0) return;   // no magnetic equation at l = 0 (Sphere_Linear_Terms.F90:160-163)
     const double llp1 = (double)l * (l + 1);
-    auto add = [&](std::vector<double>& M, int slot, int d, int i, double amp, bool stat) {
-        if (slot >= 0) coefm[(size_t)slot * nr + i] += stat ? amp : amp * rf;
-        const double fac = stat ? 1.0 : lf;
-        const double* Dd = D + (size_t)d * nr * nr;
-        for (int j = 0; j < nr; ++j) M[(size_t)i * nr + j] += amp * fac * Dd[(size_t)i * nr + j];
+    std::vector<double> amp(nr), v(nr);
+    auto add = [&](int sys, int slot, int d, bool stat) {
+        for (int i = 0; i < nr; ++i) {
+            coefm[(size_t)slot * nr + i] += stat ? amp[i] : amp[i] * rf;
+            v[i] = amp[i] * (stat ? 1.0 : lf);
+        }
+        out.add(sys, 0, 0, d, v);
     };
-    for (int i = 0; i < nr; ++i) {
-        const double H = -llp1 / (r[i] * r[i]);
-        add(Am, MS_A0, 0, i, 1.0, true);
-        add(Am, MS_A0, 0, i, H * eta[i], false);
-        add(Am, MS_A2, 2, i, 1.0 * eta[i], false);
-        add(Am, MS_A1, 1, i, c.rad.a_diff1[i], false);   // A_Diffusion_Coefs_1
-        add(Cm, MS_C0, 0, i, 1.0, true);
-        add(Cm, MS_C0, 0, i, H * eta[i], false);
-        add(Cm, MS_C2, 2, i, 1.0 * eta[i], false);
+    auto set = [&](auto f) {
+        for (int i = 0; i < nr; ++i) amp[i] = f(i);
+    };
+    for (int sys : {SYS_A, SYS_C}) {
+        set([&](int) { return 1.0; });
+        add(sys, sys == SYS_A ? MS_A0 : MS_C0, 0, true);
+        set([&](int i) { return -llp1 / (r[i] * r[i]) * eta[i]; });
+        add(sys, sys == SYS_A ? MS_A0 : MS_C0, 0, false);
+        set([&](int i) { return 1.0 * eta[i]; });
+        add(sys, sys == SYS_A ? MS_A2 : MS_C2, 2, false);
+        if (sys == SYS_A) {
+            set([&](int i) { return c.rad.a_diff1[i]; });   // A_Diffusion_Coefs_1
+            add(sys, MS_A1, 1, false);
+        }
     }
-    auto clear = [&](std::vector<double>& M, int row) {
-        std::fill(M.begin() + (size_t)row * nr, M.begin() + (size_t)(row + 1) * nr, 0.0);
-    };
-    auto bc = [&](std::vector<double>& M, int row, int d, double amp) {
-        const double* Dd = D + (size_t)d * nr * nr;
-        for (int j = 0; j < rda - 1; ++j) M[(size_t)row * nr + j] += amp * Dd[(size_t)row * nr + j];
-    };
     const int top = 0, bot = nr - 1;
-    clear(Cm, top);
-    clear(Cm, bot);
-    clear(Am, top);
-    clear(Am, bot);
-    bc(Am, top, 0, 1.0);
-    bc(Am, bot, 0, 1.0);
-    bc(Cm, top, 1, 1.0);
-    bc(Cm, top, 0, l / r[top]);
-    bc(Cm, bot, 1, 1.0);
-    bc(Cm, bot, 0, -(l + 1) / r[bot]);
+    for (int sys : {SYS_C, SYS_A}) {
+        out.clear(sys, top);
+        out.clear(sys, bot);
+    }
+    out.bc(SYS_A, top, 0, 0, 1.0);
+    out.bc(SYS_A, bot, 0, 0, 1.0);
+    out.bc(SYS_C, top, 0, 1, 1.0);
+    out.bc(SYS_C, top, 0, 0, l / r[top]);
+    out.bc(SYS_C, bot, 0, 1, 1.0);
+    out.bc(SYS_C, bot, 0, 0, -(l + 1) / r[bot]);
 }
 
 // Finalize_EMF's radial operator (Sphere_Spectral_Space.F90:436-488, Chebyshev branch) as one
@@ -495,17 +554,16 @@ static void emf_matrix(const Ctx& c, std::vector<double>& M) {
         }
 }
 
-// One l of the implicit system: LHS (row-major) and the Post_Solve RHS coefficients.
-static void build_l(const Ctx& c, int l, std::vector<double>& A, std::vector<double>& Z, double* coef) {
-    const int nr = c.d.nr, n3 = 3 * nr, rda = c.d.rda;
+// One l of the implicit system: the terms and boundary rows of the W-P-T and Z matrices, into the
+// sink, and the Post_Solve RHS coefficients.
+template <class Sink>
+static void terms_l(const Ctx& c, int l, Sink& out, double* coef) {
+    const int nr = c.d.nr, n3 = 3 * nr;
     const ra_config& cfg = c.cfg;
     const Radial& R = c.rad;
     const std::vector<double>& r = R.radius;
     const double dt = c.dt, al = cfg.alpha_implicit;
     const double lf = -dt * al, rf = dt * (1.0 - al);
-    const double* D = c.cheb_D.data();
-    A.assign((size_t)n3 * n3, 0.0);
-    Z.assign((size_t)nr * nr, 0.0);
     std::fill(coef, coef + (size_t)NSLOT * nr, 0.0);
     // slot lookup for (eq, var, d); var/d given as the grid source
     auto slot_of = [&](int eq, int var, int d) -> int {
@@ -516,23 +574,18 @@ static void build_l(const Ctx& c, int l, std::vector<double>& A, std::vector<dou
             if (kSlots[s].eq == eq && kSlots[s].g == gs) return s;
         return -1;
     };
+    std::vector<double> scaled(nr);
     // Add_Implicit_Term: LHS += amp*(static ? 1 : lf)*D_d in rows of eq, columns of var;
     // Post_Solve coefficient += amp*(static ? 1 : rf)
     auto add = [&](int eq, int var, int d, const std::vector<double>& amp, bool stat) {
         const int s = slot_of(eq, var, d);
         if (s >= 0)
             for (int i = 0; i < nr; ++i) coef[(size_t)s * nr + i] += stat ? amp[i] : amp[i] * rf;
-        const double fac = stat ? 1.0 : lf;
-        const double* Dd = D + (size_t)d * nr * nr;
-        if (eq == EQ_Z) {
-            for (int i = 0; i < nr; ++i)
-                for (int j = 0; j < nr; ++j) Z[(size_t)i * nr + j] += amp[i] * fac * Dd[(size_t)i * nr + j];
-        } else {
-            const int rb = eq * nr, cb = var * nr;
-            for (int i = 0; i < nr; ++i)
-                for (int j = 0; j < nr; ++j)
-                    A[(size_t)(rb + i) * n3 + cb + j] += amp[i] * fac * Dd[(size_t)i * nr + j];
-        }
+        for (int i = 0; i < nr; ++i) scaled[i] = amp[i] * (stat ? 1.0 : lf);
+        if (eq == EQ_Z)
+            out.add(SYS_Z, 0, 0, d, scaled);
+        else
+            out.add(SYS_WPT, eq, var, d, scaled);
     };
     std::vector<double> ones(nr, 1.0), v(nr);
     const double llp1 = (double)l * (l + 1);
@@ -580,83 +633,66 @@ static void build_l(const Ctx& c, int l, std::vector<double>& A, std::vector<dou
     }
     // Set_Boundary_Conditions (Sphere_Linear_Terms.F90:539-1100):
     // clear boundary rows, then Load_Single_Row_Cheby over the dealiased columns
-    auto clear = [&](std::vector<double>& M, int ncols, int row) {
-        std::fill(M.begin() + (size_t)row * ncols, M.begin() + (size_t)(row + 1) * ncols, 0.0);
-    };
-    auto bc = [&](std::vector<double>& M, int ncols, int row, int col0, int d, double amp) {
-        const double* Dd = D + (size_t)d * nr * nr;
-        const int rr = row % nr;
-        for (int j = 0; j < rda - 1; ++j) M[(size_t)row * ncols + col0 + j] += amp * Dd[(size_t)rr * nr + j];
-    };
     const int top = 0, bot = nr - 1;
     if (l == 0) {
-        clear(A, n3, nr + top);
-        clear(A, n3, 2 * nr + top);
-        clear(A, n3, 2 * nr + bot);
-        bc(A, n3, 2 * nr + top, 2 * nr, cfg.fix_tvar_top ? 0 : 1, 1.0);
-        bc(A, n3, 2 * nr + bot, 2 * nr, cfg.fix_tvar_bottom ? 0 : 1, 1.0);
-        bc(A, n3, nr + top, nr, 0, 1.0);   // pressure node at the top
+        out.clear(SYS_WPT, nr + top);
+        out.clear(SYS_WPT, 2 * nr + top);
+        out.clear(SYS_WPT, 2 * nr + bot);
+        out.bc(SYS_WPT, 2 * nr + top, 2 * nr, cfg.fix_tvar_top ? 0 : 1, 1.0);
+        out.bc(SYS_WPT, 2 * nr + bot, 2 * nr, cfg.fix_tvar_bottom ? 0 : 1, 1.0);
+        out.bc(SYS_WPT, nr + top, nr, 0, 1.0);   // pressure node at the top
     } else {
         for (int rb = 0; rb < n3; rb += nr) {
-            clear(A, n3, rb + top);
-            clear(A, n3, rb + bot);
+            out.clear(SYS_WPT, rb + top);
+            out.clear(SYS_WPT, rb + bot);
         }
-        clear(Z, nr, top);
-        clear(Z, nr, bot);
-        bc(A, n3, 2 * nr + top, 2 * nr, cfg.fix_tvar_top ? 0 : 1, 1.0);
-        bc(A, n3, 2 * nr + bot, 2 * nr, cfg.fix_tvar_bottom ? 0 : 1, 1.0);
-        bc(A, n3, top, 0, 0, 1.0);   // impenetrable: W = 0
-        bc(A, n3, bot, 0, 0, 1.0);
+        out.clear(SYS_Z, top);
+        out.clear(SYS_Z, bot);
+        out.bc(SYS_WPT, 2 * nr + top, 2 * nr, cfg.fix_tvar_top ? 0 : 1, 1.0);
+        out.bc(SYS_WPT, 2 * nr + bot, 2 * nr, cfg.fix_tvar_bottom ? 0 : 1, 1.0);
+        out.bc(SYS_WPT, top, 0, 0, 1.0);   // impenetrable: W = 0
+        out.bc(SYS_WPT, bot, 0, 0, 1.0);
         if (cfg.no_slip_top) {
-            bc(Z, nr, top, 0, 0, 1.0);
-            bc(A, n3, nr + top, 0, 1, 1.0);
+            out.bc(SYS_Z, top, 0, 0, 1.0);
+            out.bc(SYS_WPT, nr + top, 0, 1, 1.0);
         } else {
             const double samp = -(2.0 / r[top] + R.dlnrho[top]);
-            bc(A, n3, nr + top, 0, 2, 1.0);
-            bc(A, n3, nr + top, 0, 1, samp);
-            bc(Z, nr, top, 0, 1, 1.0);
-            bc(Z, nr, top, 0, 0, samp);
+            out.bc(SYS_WPT, nr + top, 0, 2, 1.0);
+            out.bc(SYS_WPT, nr + top, 0, 1, samp);
+            out.bc(SYS_Z, top, 0, 1, 1.0);
+            out.bc(SYS_Z, top, 0, 0, samp);
         }
         if (cfg.no_slip_bottom) {
-            bc(A, n3, nr + bot, 0, 1, 1.0);
-            bc(Z, nr, bot, 0, 0, 1.0);
+            out.bc(SYS_WPT, nr + bot, 0, 1, 1.0);
+            out.bc(SYS_Z, bot, 0, 0, 1.0);
         } else {
             const double samp = -(2.0 / r[bot] + R.dlnrho[bot]);
-            bc(A, n3, nr + bot, 0, 2, 1.0);
-            bc(A, n3, nr + bot, 0, 1, samp);
-            bc(Z, nr, bot, 0, 1, 1.0);
-            bc(Z, nr, bot, 0, 0, samp);
+            out.bc(SYS_WPT, nr + bot, 0, 2, 1.0);
+            out.bc(SYS_WPT, nr + bot, 0, 1, samp);
+            out.bc(SYS_Z, bot, 0, 1, 1.0);
+            out.bc(SYS_Z, bot, 0, 0, samp);
         }
     }
 }
 
 // Reset_Linear_Equations: build every l, upload, invert on the device.
 static void linear_setup(Ctx& c) {
-    const int L = c.d.L, nr = c.d.nr, n3 = 3 * nr;
-    std::vector<double> coef((size_t)L * NSLOT * nr);
-    std::vector<double> Aall((size_t)L * n3 * n3), Zall((size_t)L * nr * nr);
-    std::vector<double> A, Z;
+    const int L = c.d.L, nr = c.d.nr;
+    const size_t na = (size_t)L * AsmShape::MAXT * nr, nb = (size_t)L * AsmShape::MAXB;
+    std::vector<double> coef((size_t)L * NSLOT * nr), cm(c.mag ? (size_t)L * NMSLOT * nr : 0), amp(na + nb);
+    AsmShape shape[2];
     for (int l = 0; l < L; ++l) {
-        build_l(c, l, A, Z, coef.data() + (size_t)l * NSLOT * nr);
-        std::copy(A.begin(), A.end(), Aall.begin() + (size_t)l * n3 * n3);
-        std::copy(Z.begin(), Z.end(), Zall.begin() + (size_t)l * nr * nr);
+        RecipeSink out(amp.data() + (size_t)l * AsmShape::MAXT * nr, amp.data() + na + (size_t)l * AsmShape::MAXB, nr);
+        terms_l(c, l, out, coef.data() + (size_t)l * NSLOT * nr);
+        if (c.mag) terms_l_mag(c, l, out, cm.data() + (size_t)l * NMSLOT * nr);
+        if (l < 2) shape[l] = out.S;
     }
+    if (!c.d_asm) RA_CUDA(cudaMalloc(&c.d_asm, (na + nb) * sizeof(double)));
+    RA_CUDA(cudaMemcpyAsync(c.d_asm, amp.data(), (na + nb) * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     RA_CUDA(cudaMemcpyAsync(c.d_coef, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    RA_CUDA(cudaMemcpyAsync(c.d_Awpt, Aall.data(), Aall.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    RA_CUDA(cudaMemcpyAsync(c.d_Az, Zall.data(), Zall.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    if (c.mag) {
-        std::vector<double> cm((size_t)L * NMSLOT * nr), Call((size_t)L * nr * nr), Aall2((size_t)L * nr * nr);
-        std::vector<double> Cm, Am;
-        for (int l = 0; l < L; ++l) {
-            build_l_mag(c, l, Cm, Am, cm.data() + (size_t)l * NMSLOT * nr);
-            std::copy(Cm.begin(), Cm.end(), Call.begin() + (size_t)l * nr * nr);
-            std::copy(Am.begin(), Am.end(), Aall2.begin() + (size_t)l * nr * nr);
-        }
+    if (c.mag)
         RA_CUDA(cudaMemcpyAsync(c.d_coef_mag, cm.data(), cm.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        RA_CUDA(cudaMemcpyAsync(c.d_Ac, Call.data(), Call.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        RA_CUDA(cudaMemcpyAsync(c.d_Aa, Aall2.data(), Aall2.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-        RA_CUDA(cudaStreamSynchronize(c.stream));   // the host vectors go out of scope
-    }
+    launch_assemble(c, shape[0], shape[1], c.d_asm, c.d_asm + na);
     factor_matrices(c);
 }
 
@@ -916,7 +952,7 @@ static void release(Ctx& c) {
     if (c.d_adapt) cudaFree(c.d_adapt);
     if (c.d_adapt_dt) cudaFree(c.d_adapt_dt);
     lu_workspace_free(c.lu_work);
-    double* bufs[] = {c.d_Ptab, c.d_iPtab, c.d_D, c.d_Dpar, c.d_Dfd, c.d_coef, c.d_radial, c.d_costh, c.d_twid, c.d_twp, c.d_twq,
+    double* bufs[] = {c.d_Ptab, c.d_iPtab, c.d_D, c.d_Dpar, c.d_Dfd, c.d_coef, c.d_radial, c.d_costh, c.d_twid, c.d_twp, c.d_twq, c.d_asm,
                       c.d_Awpt, c.d_Az,
                       c.d_Ainv_wpt, c.d_Ainv_z,
                       c.d_sol_wpt, c.d_sol_z, c.d_rhs_wpt, c.d_rhs_z, c.d_ab, c.d_g, c.d_s2a, c.d_s2a11,
@@ -1592,22 +1628,21 @@ int ra_build_matrices(const ra_config* cfg, int sys, int l0, int nl, double* lhs
         radial_setup(c, rmax * cfg->aspect_ratio, rmax);
         reference_setup(c);
         const int nr = c.d.nr, n = sys ? nr : 3 * nr;
-        std::vector<double> A, Z, cf((size_t)NSLOT * nr), cm((size_t)NMSLOT * nr);
+        std::vector<double> cf((size_t)NSLOT * nr), cm((size_t)NMSLOT * nr);
+        MatrixSink sink(c);
         // coefficient slots of the magnetic systems: C (C,C,0) (C,C,2); A (A,A,0) (A,A,1) (A,A,2)
         static const int kMagSlots[2][3] = {{MS_C0, MS_C2, -1}, {MS_A0, MS_A1, MS_A2}};
         for (int i = 0; i < nl; ++i) {
-            const std::vector<double>* M;
-            if (sys < 2) {
-                build_l(c, l0 + i, A, Z, cf.data());
-                M = sys ? &Z : &A;
-            } else {
-                build_l_mag(c, l0 + i, Z, A, cm.data());   // Z: C, A: A
-                M = sys == 2 ? &Z : &A;
-            }
+            sink.begin();
+            if (sys < 2)
+                terms_l(c, l0 + i, sink, cf.data());
+            else
+                terms_l_mag(c, l0 + i, sink, cm.data());
+            const std::vector<double>& M = sink.M[sys];
             if (lhs) {
                 double* out = lhs + (size_t)i * n * n;   // column-major
                 for (int r = 0; r < n; ++r)
-                    for (int k = 0; k < n; ++k) out[(size_t)k * n + r] = (*M)[(size_t)r * n + k];
+                    for (int k = 0; k < n; ++k) out[(size_t)k * n + r] = M[(size_t)r * n + k];
             }
             if (coefs && sys < 2) std::copy(cf.begin(), cf.end(), coefs + (size_t)i * NSLOT * nr);
             if (coefs && sys >= 2) {

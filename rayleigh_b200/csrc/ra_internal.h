@@ -144,6 +144,16 @@ struct UnitPlan {
     int ncol = 0;
 };
 
+// The terms and boundary rows of one l's matrices (k_assemble.cu): term q adds profile q times D_d to
+// the rows of eq in the columns of var of system sys; boundary rows are cleared and take their own.
+struct AsmShape {
+    static constexpr int MAXT = 40, MAXB = 24;
+    int nterm, nclear, nbc;
+    signed char sys[MAXT], eq[MAXT], var[MAXT], d[MAXT];
+    signed char clear_sys[MAXB], bc_sys[MAXB], bc_d[MAXB];
+    int clear_row[MAXB], bc_row[MAXB], bc_col[MAXB];
+};
+
 struct Ctx {
     ra_config cfg;
     Dims d;
@@ -174,6 +184,7 @@ struct Ctx {
     double *d_Ptab = nullptr, *d_iPtab = nullptr;     // [row][nth2]
     double *d_D = nullptr;                            // [4][nr][nr]
     double *d_Dpar = nullptr;                         // [4][2][nr/2][(kc+1)/2] parity planes of D, r < nr/2
+    double *d_asm = nullptr;                          // profiles and boundary amplitudes of the implicit matrices
     double *d_Dfd = nullptr;                          // finite differences: I, D1, D2, D3, D1 D1 in bands:
     int fd_w = 0;                                     //   [5][nr][1 + fd_w] = first column, fd_w coefficients
     double *d_coef = nullptr;                         // [L][NSLOT][nr]
@@ -250,6 +261,7 @@ enum { R_RADIUS, R_OVER_R, R_DELTA_R, R_DENSITY, R_DLNRHO, R_OVER_RHOR, R_OVER_R
        R_OVER_RSQ, R_VISC_HEAT, R_OHM_HEAT, R_RHO_T, R_COUNT };   // R_RHO_T: rho T of the reference state
 
 // ---- kernels / launchers (defined in the .cu files) ----
+void launch_assemble(Ctx& c, const AsmShape& s0, const AsmShape& s1, const double* d_amp, const double* d_bamp);
 void launch_plm(Ctx& c, const double* d_x, const double* d_w);
 void launch_lt_inverse(Ctx& c, const double* s2, double* p2, int ncol);
 void launch_lt_forward(Ctx& c, const double* p2, double* s2, int ncol);
