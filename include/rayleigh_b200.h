@@ -39,7 +39,8 @@ extern "C" {
 #define RA_ERR_NONFINITE   -6   /* NaN/Inf in an input, or reaching the implicit solve during a step */
 
 #define RA_PREC_FP64   0        /* every product in FP64 */
-#define RA_PREC_MIXED  1        /* split-precision tensor-core products, FP64 state */
+#define RA_PREC_MIXED  1        /* split-precision tensor-core products, FP64 state (Legendre products of a
+                                   small l_max stay FP64: they are faster there) */
 
 typedef struct ra_ctx ra_ctx;
 
@@ -556,7 +557,8 @@ int ra_fft_c2r(ra_ctx* ctx, double* x, long howmany);
  * (Fourier_Transform.F90:142-183) in place; direction 1 (physical -> spectral) runs the r2c
  * in place on d_grid (overwriting it), folds into d_work and runs PtS_4d_dgpv3 (:1077-1175)
  * into d_spec.  precision RA_PREC_FP64 (FP64 tensor-core products) or RA_PREC_MIXED
- * (split int8 products; their plan is built on the first call with given operands).
+ * (split int8 products, where l_max is large enough for them to be the faster ones: from 199 on
+ * spectral -> physical, from 149 on back; their plan is built on the first call with given operands).
  *   d_spec: [n_lm rows][nfr][re, im], rows m-major with the even l - m first (the row order
  *           of the ra_* device buffers: row(m, l) = off(m) + (l - m even ? (l - m)/2 :
  *           ne(m) + (l - m - 1)/2), off(m) = m L - m (m - 1)/2, ne(m) = (L - m + 1)/2)

@@ -56,6 +56,12 @@ static void run_split_once(Ctx& c, const std::vector<OzSplitJob>& jobs, int max_
 // ---------------------------------------------------------------------------
 // Inverse Legendre transform
 // ---------------------------------------------------------------------------
+// Whether the mixed form's Legendre products are split products.  On small grids the digit split and
+// the product's short K cost more than the FP64 products, which are the more exact anyway: per step
+// at N_r = 64 with B, FP64 / split, the inverse takes 51 / 115 us at l_max = 63, 250 / 301 at 127 and
+// 441 / 610 at 170, but 1263 / 1009 at 255; the forward 35 / 67, 113 / 147, 230 / 209 and 598 / 423.
+bool lt_split(const Ctx& c, bool inverse) { return c.d.L >= (inverse ? 200 : 150); }
+
 // The plan of one batched inverse transform p2 = P s2 over ncol columns (s2 rows in the
 // m-major parity-sorted order, p2[theta_h][m][par][col]): the step's (s2a11 -> p2a) and the
 // device-resident unit transform's.
@@ -299,8 +305,8 @@ void mixed_setup(Ctx& c) {
         malloc_dev(c.d_status, 1);
         RA_CUDA(cudaMemsetAsync(c.d_status, 0, sizeof(int), c.stream));
     }
-    setup_lt_inverse(c);
-    setup_lt_forward(c);
+    if (lt_split(c, true)) setup_lt_inverse(c);
+    if (lt_split(c, false)) setup_lt_forward(c);
     if (c.mixed_solve) setup_solve(c);
 }
 

@@ -995,7 +995,7 @@ static void run_stage(Ctx& c, int k, double new_ab, double old_ab) {
             launch_rlm_a(c);   // with the magnetic fields when c.mag
             break;
         case 3:
-            if (mixed)
+            if (mixed && lt_split(c, true))
                 launch_lt_inverse_mixed(c);
             else
                 launch_lt_inverse(c, c.d_s2a11, c.d_p2a, c.nfa * c.d.nr * 2);
@@ -1005,7 +1005,7 @@ static void run_stage(Ctx& c, int k, double new_ab, double old_ab) {
             launch_physics(c);
             break;
         case 5:
-            if (mixed)
+            if (mixed && lt_split(c, false))
                 launch_lt_forward_mixed(c);
             else
                 launch_lt_forward(c, c.d_p2b, c.d_s2b, c.nfb * c.d.nr * 2);

@@ -341,6 +341,7 @@ void launch_fft_rows(Ctx& c, double* d_x, long howmany, int inverse);
 void launch_cheb_columns(Ctx& c, const double* d_in, double* d_out, long ncols, int mode, int order);
 void mixed_setup(Ctx& c);
 void mixed_release(Ctx& c);
+bool lt_split(const Ctx& c, bool inverse);
 void launch_lt_inverse_mixed(Ctx& c);
 void launch_lt_unit_mixed(Ctx& c, int inverse, const double* in, double* out, int ncol);
 void transform_dev(Ctx& c, int direction, int precision, double* spec, double* grid, double* work, int nfr,

@@ -95,13 +95,14 @@ void transform_dev(Ctx& c, int direction, int precision, double* spec, double* g
     cudaEvent_t ev[4];
     for (auto& e : ev) RA_CUDA(cudaEventCreate(&e));
     auto product = [&] {
+        const bool split = precision == RA_PREC_MIXED && lt_split(c, direction == 0);
         if (direction == 0) {
-            if (precision == RA_PREC_MIXED)
+            if (split)
                 launch_lt_unit_mixed(c, 1, spec, work, ncol);
             else
                 launch_lt_inverse(c, spec, work, ncol);
         } else {
-            if (precision == RA_PREC_MIXED)
+            if (split)
                 launch_lt_unit_mixed(c, 0, work, spec, ncol);
             else
                 launch_lt_forward(c, work, spec, ncol);
