@@ -13,7 +13,7 @@
 //  All m share one launch; K (the number of l of one parity) is ragged and the
 //  grid is ordered by m so that the long products start first.
 #include "ra_internal.h"
-#include "gemm_f64.cuh"
+#include "gemm_async.cuh"
 
 namespace ra {
 
@@ -139,43 +139,45 @@ void launch_plm(Ctx& c, const double* d_x, const double* d_w) {
 // theta_h is the slowest index so that the physical-space kernel, which reads
 // every (m, parity) of one theta_h, touches one contiguous block.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(GEMM_THREADS) lt_inverse_kernel(const double* __restrict__ Ptab,
-                                                                  const double* __restrict__ s2,
-                                                                  double* __restrict__ p2, int L, int nth,
-                                                                  int ncol) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    GemmSmem& sm = *reinterpret_cast<GemmSmem*>(smem_raw);
+template <bool VEC>
+__global__ void __launch_bounds__(GEMM_THREADS, 4) lt_inverse_kernel(const double* __restrict__ Ptab,
+                                                                     const double* __restrict__ s2,
+                                                                     double* __restrict__ p2, int L, int nth,
+                                                                     int ncol) {
+    using OA = OperandX<true, 4>;
+    using OB = OperandX<VEC, 4>;
+    extern __shared__ __align__(16) double ga_sm[];
     const int m = blockIdx.z >> 1, par = blockIdx.z & 1;
-    const int th0 = blockIdx.y * BM;
-    const int c0 = blockIdx.x * BN;
+    const int th0 = blockIdx.y * GA_BM;
+    const int c0 = blockIdx.x * GA_BN;
     const int nth2 = nth / 2;
     const int ne = n_even(m, L);
     const int nl = par ? n_odd(m, L) : ne;
     const long roff = m_off(m, L) + (par ? ne : 0);
-    const double* pa = Ptab + roff * nth2;
-    const double* pb = s2 + roff * ncol;
     Acc acc;
     acc.zero();
-    auto fa = [&](int k, int x) -> double {
-        const int th = th0 + x;
-        return (k < nl && th < nth2) ? __ldg(pa + (long)k * nth2 + th) : 0.0;
-    };
-    auto fb = [&](int k, int y) -> double {
-        const int col = c0 + y;
-        return (k < nl && col < ncol) ? __ldg(pb + (long)k * ncol + col) : 0.0;
-    };
-    gemm_tile<true, true>(acc, fa, fb, nl, sm);
-    double* out = p2 + (long)blockIdx.z * ncol;
+    gemm_async<false>(acc, OA{Ptab + roff * nth2 + th0, nth2, nl, nth2 - th0}, OB{s2 + roff * ncol + c0, ncol, nl, ncol - c0},
+                      nl, ga_sm);
+    double* out = p2 + (long)blockIdx.z * ncol + c0;
     const long th_stride = 2L * L * ncol;
-    acc_foreach(acc, [&](int x, int y, double v) {
-        const int th = th0 + x, col = c0 + y;
-        if (th < nth2 && col < ncol) out[(long)th * th_stride + col] = v;
+    acc_each<false>(acc, [&](int x, int y, double v0, double v1) {
+        if (th0 + x < nth2 && c0 + y < ncol)
+            *reinterpret_cast<double2*>(out + (long)(th0 + x) * th_stride + y) = make_double2(v0, v1);
     });
 }
 
+// n_theta / 2 and ncol are even, the tables and p2 16-byte aligned (p2 is read as complex values); a
+// caller's coefficients may be 8-byte aligned only.
 void launch_lt_inverse(Ctx& c, const double* s2, double* p2, int ncol) {
-    dim3 grid((ncol + BN - 1) / BN, (c.d.nth2 + BM - 1) / BM, 2 * c.d.L);
-    lt_inverse_kernel<<<grid, GEMM_THREADS, sizeof(GemmSmem), c.stream>>>(c.d_Ptab, s2, p2, c.d.L, c.d.nth, ncol);
+    dim3 grid((ncol + GA_BN - 1) / GA_BN, (c.d.nth2 + GA_BM - 1) / GA_BM, 2 * c.d.L);
+    auto go = [&](auto kern, size_t sm) {
+        RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        kern<<<grid, GEMM_THREADS, sm, c.stream>>>(c.d_Ptab, s2, p2, c.d.L, c.d.nth, ncol);
+    };
+    if ((reinterpret_cast<uintptr_t>(s2) & 15) == 0)
+        go(lt_inverse_kernel<true>, ga_smem<OperandX<true, 4>, OperandX<true, 4>>());
+    else
+        go(lt_inverse_kernel<false>, ga_smem<OperandX<true, 4>, OperandX<false, 4>>());
     RA_CUDA(cudaGetLastError());
     ++c.launches;
 }
@@ -186,36 +188,38 @@ void launch_lt_inverse(Ctx& c, const double* s2, double* p2, int ncol) {
 //   s2[row(m, l)][col] = sum_th iP_par(l, th) p2[m][par][th][col]
 // tiles: (m, parity, l-tile) in descending-K order
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(GEMM_THREADS) lt_forward_kernel(const double* __restrict__ iPtab,
-                                                                  const double* __restrict__ p2,
-                                                                  double* __restrict__ s2,
-                                                                  const int4* __restrict__ tiles, int L,
-                                                                  int nth, int ncol) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    GemmSmem& sm = *reinterpret_cast<GemmSmem*>(smem_raw);
+using FwdA = OperandK;
+using FwdB = OperandX<true, 2>;   // rows 2 tig apart: 528-byte rows keep a fragment phase conflict-free
+
+template <bool VEC>
+__global__ void __launch_bounds__(GEMM_THREADS, 4) lt_forward_kernel(const double* __restrict__ iPtab,
+                                                                     const double* __restrict__ p2,
+                                                                     double* __restrict__ s2,
+                                                                     const int4* __restrict__ tiles, int L,
+                                                                     int nth, int ncol) {
+    extern __shared__ __align__(16) double ga_sm[];
     const int4 tl = tiles[blockIdx.y];
-    const int m = tl.x, par = tl.y, l0 = tl.z * BM;
-    const int c0 = blockIdx.x * BN;
+    const int m = tl.x, par = tl.y, l0 = tl.z * GA_BM;
+    const int c0 = blockIdx.x * GA_BN;
     const int nth2 = nth / 2;
     const int ne = n_even(m, L);
     const int nl = par ? n_odd(m, L) : ne;
     const long roff = m_off(m, L) + (par ? ne : 0) + l0;
-    const double* pa = iPtab + roff * nth2;
-    const double* pm = p2 + ((long)m * 2 + par) * nth2 * ncol;
     Acc acc;
     acc.zero();
-    auto fa = [&](int k, int x) -> double {
-        return (l0 + x < nl && k < nth2) ? __ldg(pa + (long)x * nth2 + k) : 0.0;
-    };
-    auto fb = [&](int k, int y) -> double {
-        const int col = c0 + y;
-        return (k < nth2 && col < ncol) ? __ldg(pm + (long)k * ncol + col) : 0.0;
-    };
-    gemm_tile<false, true>(acc, fa, fb, nth2, sm);
-    double* out = s2 + roff * ncol;
-    acc_foreach(acc, [&](int x, int y, double v) {
-        const int col = c0 + y;
-        if (l0 + x < nl && col < ncol) out[(long)x * ncol + col] = v;
+    gemm_async<true>(acc, FwdA{iPtab + roff * nth2, nth2, nth2, nl - l0},
+                     FwdB{p2 + ((long)m * 2 + par) * nth2 * ncol + c0, ncol, nth2, ncol - c0}, nth2, ga_sm);
+    double* out = s2 + roff * ncol + c0;
+    acc_each<true>(acc, [&](int x, int y, double v0, double v1) {
+        if (l0 + x < nl && c0 + y < ncol) {
+            double* o = out + (long)x * ncol + y;
+            if constexpr (VEC) {
+                *reinterpret_cast<double2*>(o) = make_double2(v0, v1);
+            } else {
+                o[0] = v0;
+                o[1] = v1;
+            }
+        }
     });
 }
 
@@ -224,7 +228,7 @@ static std::vector<int> forward_tiles(int L) {
     for (int m = 0; m < L; ++m) {
         for (int par = 0; par < 2; ++par) {
             const int nl = par ? n_odd(m, L) : n_even(m, L);
-            for (int lt = 0; lt * BM < nl; ++lt) {
+            for (int lt = 0; lt * GA_BM < nl; ++lt) {
                 t.push_back(m);
                 t.push_back(par);
                 t.push_back(lt);
@@ -248,9 +252,17 @@ void lt_forward_prepare(Ctx& c) {
 
 void launch_lt_forward(Ctx& c, const double* p2, double* s2, int ncol) {
     if (!c.d_fwd_tiles) throw ArgError("forward-transform tiles not prepared (lt_forward_prepare runs at set-up)");
-    dim3 grid((ncol + BN - 1) / BN, c.n_fwd_tiles);
-    lt_forward_kernel<<<grid, GEMM_THREADS, sizeof(GemmSmem), c.stream>>>(
-        c.d_iPtab, p2, s2, reinterpret_cast<const int4*>(c.d_fwd_tiles), c.d.L, c.d.nth, ncol);
+    dim3 grid((ncol + GA_BN - 1) / GA_BN, c.n_fwd_tiles);
+    const size_t sm = ga_smem<FwdA, FwdB>();
+    auto go = [&](auto kern) {
+        RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        kern<<<grid, GEMM_THREADS, sm, c.stream>>>(c.d_iPtab, p2, s2, reinterpret_cast<const int4*>(c.d_fwd_tiles),
+                                                   c.d.L, c.d.nth, ncol);
+    };
+    if ((reinterpret_cast<uintptr_t>(s2) & 15) == 0)
+        go(lt_forward_kernel<true>);
+    else
+        go(lt_forward_kernel<false>);
     RA_CUDA(cudaGetLastError());
     ++c.launches;
 }
