@@ -29,39 +29,46 @@ __device__ __forceinline__ int ell_of_lm(long lm) {
 // Chebyshev synthesis of the 12 grid outputs (W W' W'' W''' P P' T T' T'' Z Z' Z'')
 // ---------------------------------------------------------------------------
 
-// One CTA per (field, 128-column tile).  D(n_r - 1 - r, k) = (-1)^(k+d) D(r, k),
-// so rows r < n_r/2 give both halves of the grid:
+// D(n_r - 1 - r, k) = (-1)^(k+d) D(r, k), so rows r < n_r/2 give both halves of the grid:
 //   g(r) = E + O,  g(n_r - 1 - r) = (-1)^d (E - O),
-// E / O the products over even / odd k.  Dpar[d][par][r][k'] = D_d(r, 2k' + par).
-// Per (derivative order, 32-row block: the n_r/2 = 96 half-grid rows in three
-// full blocks) the CTA computes E, parks it in shared memory (each thread its
-// own accumulator slots, so no barrier), computes O in the same registers and
-// writes both halves.  The coefficients stream through the tile engine's own
-// double-buffered stage from L2: one accumulator and no coefficient stage keep
-// a CTA at about 75 KB of shared memory and 168 registers, three CTAs per SM.
+// E / O the products over even / odd k.  One CTA per (field, 64 columns): the columns'
+// coefficients (k < kc, the rest zero) sit in shared memory for every derivative order and row
+// block, the rows of D stream through a three-stage cp.async ring that runs on over the blocks,
+// and E and O accumulate side by side: a 16-byte fragment at k = 2 k' holds the even and the odd
+// value, of D as of the coefficients.
+// What bounds it: the FP64 tensor pipe and, a little below it, the writes of the grids.  The form that
+// streamed the coefficients anew for every order, row block and parity (products only four
+// k-steps long, each started from an empty pipe) ran at 0.44 of the DGEMM rate.
 struct ChebField { int o0, nd, var; };
 __constant__ ChebField kChebField[6] = {{G_W0, 4, 0}, {G_P0, 2, 1}, {G_T0, 3, 2}, {G_Z0, 3, 3},
                                         {G_C0, 3, 4}, {G_A0, 3, 5}};   // C and A with magnetism
 
-using ChebShape = Wide;   // 32 x 128 tiles: 32-row blocks cover the n_r/2 = 96 half-grid rows exactly
-struct ChebSmem {
-    GemmSmemT<1, 4> g;
-    double park[32][GEMM_THREADS];   // E of the thread's 32 accumulator slots
-};
+constexpr int CH_COLS = 64, CH_ROWS = 32, CH_K = 32, CH_STAGES = 3, CH_THREADS = 128;
+constexpr int CH_LDA = CH_K + 8;   // row strides of 8 mod 16 doubles: the two rows of a fragment phase
+                                   // lie in different halves of the banks
+__host__ __device__ constexpr int cheb_ldb(int kc) { return (kc + CH_K - 1) / CH_K * CH_K + 8; }
 
-__global__ void __launch_bounds__(GEMM_THREADS, 3) cheb_synthesis_kernel(const double* __restrict__ Dpar,
-                                                                         const double* __restrict__ sol_wpt,
-                                                                         const double* __restrict__ sol_z,
-                                                                         const double* __restrict__ sol_c,
-                                                                         const double* __restrict__ sol_a,
-                                                                         double* __restrict__ g, int nr, int kc,
-                                                                         long ncols) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    ChebSmem& sm = *reinterpret_cast<ChebSmem*>(smem_raw);
-    const int kh = (kc + 1) / 2;   // coefficients per parity (the odd plane has one fewer when kc is odd)
+// 16 bytes, of which the first `bytes` come from src and the rest are zero
+__device__ __forceinline__ void cheb_copy(double* dst, const double* src, int bytes) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(src), "r"(bytes) : "memory");
+}
+
+__global__ void __launch_bounds__(CH_THREADS, 3) cheb_synthesis_kernel(const double* __restrict__ D,
+                                                                       const double* __restrict__ sol_wpt,
+                                                                       const double* __restrict__ sol_z,
+                                                                       const double* __restrict__ sol_c,
+                                                                       const double* __restrict__ sol_a,
+                                                                       double* __restrict__ g, int nr, int kc,
+                                                                       long ncols) {
+    extern __shared__ __align__(16) double ch_sm[];
+    const int ldb = cheb_ldb(kc), nch = (kc + CH_K - 1) / CH_K;
+    double* Bs = ch_sm;                      // [CH_COLS][ldb]
+    double* As = Bs + CH_COLS * ldb;         // [CH_STAGES][CH_ROWS][CH_LDA]
     const ChebField cf = kChebField[blockIdx.y];
-    const long c0 = (long)blockIdx.x * ChebShape::BN;
-    const int nr2 = nr / 2;
+    if ((int)blockIdx.z >= cf.nd) return;
+    const long c0 = (long)blockIdx.x * CH_COLS;
+    const int nr2 = nr / 2, nrb = (nr2 + CH_ROWS - 1) / CH_ROWS;
     const double* src;
     long cstride;
     if (cf.var < 3) {
@@ -72,47 +79,90 @@ __global__ void __launch_bounds__(GEMM_THREADS, 3) cheb_synthesis_kernel(const d
         cstride = nr;
     }
     const int t = threadIdx.x;
-    for (int dd = 0; dd < cf.nd; ++dd) {
-        const int o = cf.o0 + dd;
-        const double sgn = (dd & 1) ? -1.0 : 1.0;
-        double* out = g + (long)o * ncols * nr;
-        for (int r0 = 0; r0 < nr2; r0 += ChebShape::BM) {
-            Acc acc;
-#pragma unroll 1
-            for (int par = 0; par < 2; ++par) {
-                const double* Dp = Dpar + (((long)dd * 2 + par) * nr2) * kh;
-                auto fa = [&](int k, int x) -> double {
-                    const int r = r0 + x;
-                    return (k < kh && r < nr2) ? __ldg(Dp + (long)r * kh + k) : 0.0;
-                };
-                auto fb = [&](int k, int y) -> double {   // coefficient 2k + par of column c0 + y
-                    const long col = c0 + y;
-                    const int kk = 2 * k + par;
-                    return (kk < kc && col < ncols) ? __ldg(src + col * cstride + kk) : 0.0;
-                };
-                acc.zero();
-                gemm_tile<false, false, 1, 4>(acc, fa, fb, kh, sm.g);
-                if (par == 0) {
+    const int lane = t & 31, warp = t >> 5, gg = lane >> 2, tig = lane & 3;
+    auto bytes_at = [&](int kk) { return kk + 1 < kc ? 16 : (kk < kc ? 8 : 0); };
+    // the rows of D in order: derivative order, row block, k chunk
+    int f_dd = blockIdx.z, f_rb = 0, f_ch = 0, f_stage = 0;
+    auto fetch = [&] {
+        if (f_dd < cf.nd) {
+            double* tile = As + f_stage * CH_ROWS * CH_LDA;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-#pragma unroll
-                            for (int q = 0; q < 2; ++q) sm.park[(i * 4 + j) * 2 + q][t] = acc.v[i][j][q];
+            for (int i = 0; i < CH_ROWS * CH_K / 2 / CH_THREADS; ++i) {
+                const int e = t + i * CH_THREADS, x = e / (CH_K / 2), k = (e % (CH_K / 2)) * 2;
+                const int r = f_rb * CH_ROWS + x, kk = f_ch * CH_K + k;
+                const int bytes = r < nr2 ? bytes_at(kk) : 0;
+                cheb_copy(tile + x * CH_LDA + k, bytes ? D + ((long)f_dd * nr + r) * nr + kk : D, bytes);
+            }
+            f_stage = f_stage + 1 == CH_STAGES ? 0 : f_stage + 1;
+            if (++f_ch == nch) {
+                f_ch = 0;
+                if (++f_rb == nrb) {
+                    f_rb = 0;
+                    f_dd += gridDim.z;
                 }
             }
-            int slot = 0;
-            acc_foreach<1, 4>(acc, [&](int x, int y, double od) {
-                const double e = sm.park[slot++][t];
-                const int r = r0 + x;
-                const long col = c0 + y;
-                if (r < nr2 && col < ncols) {
-                    out[col * nr + r] = e + od;
-                    out[col * nr + (nr - 1 - r)] = sgn * (e - od);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    for (int e = t; e < CH_COLS * nch * (CH_K / 2); e += CH_THREADS) {
+        const int x = e / (nch * (CH_K / 2)), kk = (e - x * (nch * (CH_K / 2))) * 2;
+        const int bytes = c0 + x < ncols ? bytes_at(kk) : 0;
+        cheb_copy(Bs + x * ldb + kk, bytes ? src + (c0 + x) * cstride + kk : D, bytes);
+    }
+#pragma unroll
+    for (int s = 0; s < CH_STAGES - 1; ++s) fetch();   // the first group holds the coefficients too
+    int stage = 0;
+    for (int dd = blockIdx.z; dd < cf.nd; dd += gridDim.z) {
+        const double sgn = (dd & 1) ? -1.0 : 1.0;
+        double* out = g + (long)(cf.o0 + dd) * ncols * nr;
+        for (int rb = 0; rb < nrb; ++rb) {
+            const int r0 = rb * CH_ROWS, ni = min(4, (nr2 - r0 + 7) / 8);
+            double ev[4][2][2] = {}, od[4][2][2] = {};
+            for (int ch = 0; ch < nch; ++ch) {
+                asm volatile("cp.async.wait_group %0;\n" ::"n"(CH_STAGES - 2) : "memory");
+                __syncthreads();
+                fetch();
+                const double* a_t = As + stage * CH_ROWS * CH_LDA;
+                const double* b_t = Bs + (warp * 16 + gg) * ldb + ch * CH_K;
+                stage = stage + 1 == CH_STAGES ? 0 : stage + 1;
+#pragma unroll
+                for (int k = 0; k < CH_K; k += 8) {   // four k' a step
+                    double2 a[4], b[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) b[j] = *reinterpret_cast<const double2*>(b_t + j * 8 * ldb + k + 2 * tig);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        a[i] = *reinterpret_cast<const double2*>(a_t + (i * 8 + gg) * CH_LDA + k + 2 * tig);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i < ni)
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                dmma(ev[i][j], a[i].x, b[j].x);
+                                dmma(od[i][j], a[i].y, b[j].y);
+                            }
                 }
-            });
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const long col = c0 + warp * 16 + j * 8 + 2 * tig + q;
+                    if (col < ncols) {
+                        double* o = out + col * nr;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int r = r0 + i * 8 + gg;
+                            if (r < nr2) {
+                                o[r] = ev[i][j][q] + od[i][j][q];
+                                o[nr - 1 - r] = sgn * (ev[i][j][q] - od[i][j][q]);
+                            }
+                        }
+                    }
+                }
         }
     }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
 // The finite-difference radial mode's synthesis: the state holds grid values, and every grid
@@ -188,12 +238,15 @@ void launch_cheb_synthesis(Ctx& c) {
         return;
     }
     const long ncols = 2 * c.d.nlm;
-    const size_t smem = sizeof(ChebSmem);
+    const size_t smem = ((size_t)CH_COLS * cheb_ldb(c.d.kc) + CH_STAGES * CH_ROWS * CH_LDA) * sizeof(double);
     // the limit is per device: set it on every launch (a host-side call, also legal during capture)
     RA_CUDA(cudaFuncSetAttribute(cheb_synthesis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    dim3 grid((unsigned)((ncols + ChebShape::BN - 1) / ChebShape::BN), c.mag ? 6 : 4);
-    cheb_synthesis_kernel<<<grid, GEMM_THREADS, smem, c.stream>>>(c.d_Dpar, c.d_sol_wpt, c.d_sol_z, c.d_sol_c,
-                                                                   c.d_sol_a, c.d_g, c.d.nr, c.d.kc, ncols);
+    // Where the (tile, field) CTAs leave SMs without three of them, the derivative orders go to CTAs of
+    // their own: the chain of up to four orders is what a small grid waits for.
+    dim3 grid((unsigned)((ncols + CH_COLS - 1) / CH_COLS), c.mag ? 6 : 4);
+    if (grid.x * grid.y < 3 * 148) grid.z = 4;
+    cheb_synthesis_kernel<<<grid, CH_THREADS, smem, c.stream>>>(c.d_D, c.d_sol_wpt, c.d_sol_z, c.d_sol_c, c.d_sol_a,
+                                                                c.d_g, c.d.nr, c.d.kc, ncols);
     RA_CUDA(cudaGetLastError());
     ++c.launches;
 }
