@@ -129,11 +129,11 @@ __global__ void __launch_bounds__(G* M / 4) rows_r2c_kernel(PhysParams P, double
     }
     __syncthreads();
     pair_mid_pass<M, ROW_NB, S::R2, 4 * S::R2, true>(buf, P.twq + S::TW2, tt);
-    __syncthreads();
     if constexpr (S::R1 > 1) {
+        mid_barrier<M>(tt);
         pair_mid_pass<M, ROW_NB, S::R1, Q, true>(buf, P.twq, tt);
-        __syncthreads();
     }
+    __syncthreads();
     const size_t mstride = (size_t)NTH * nfr * 2, pstride = mstride / 2;   // p2[m][par][theta_h][fr]
 #pragma unroll 1
     for (int q = tt; q < NITEM; q += T) {

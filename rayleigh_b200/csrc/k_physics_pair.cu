@@ -28,11 +28,11 @@ __device__ __forceinline__ void pair_r2c(const PhysParams& P, double* __restrict
     constexpr int F = S::F, Q = S::Q, T = S::T, NITEM = NB * (Q / 2);
     __syncthreads();
     pair_mid_pass<M, NB, S::R2, 4 * S::R2, true>(buf, P.twq + S::TW2, tt);
-    __syncthreads();
     if constexpr (S::R1 > 1) {
+        mid_barrier<M>(tt);
         pair_mid_pass<M, NB, S::R1, Q, true>(buf, P.twq, tt);
-        __syncthreads();
     }
+    __syncthreads();
 #pragma unroll 1
     for (int q = tt; q < NITEM; q += T) {
         int k, b;

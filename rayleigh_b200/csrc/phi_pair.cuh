@@ -166,6 +166,18 @@ __device__ __forceinline__ void pair_mid_pass(double2* __restrict__ buf, const d
     }
 }
 
+// Barrier between the two mid passes.  Where each half of the row's threads works on its own fields in
+// both of them (two radix-8 passes: a field has T/2 butterflies) a half waits for itself only.
+template <int M>
+__device__ __forceinline__ void mid_barrier(int tt) {
+    constexpr int T = Pair<M>::T;
+    if constexpr (Pair<M>::R1 == 8 && Pair<M>::R2 == 8 && T % 64 == 0) {
+        asm volatile("bar.sync %0, %1;" ::"r"(tt < T / 2 ? 1 : 2), "r"(T / 2) : "memory");
+    } else {
+        __syncthreads();
+    }
+}
+
 // c2r of NB fields of this row pair (fields fo[b], d/dphi where dp[b]); on return y[b][i] holds the
 // (south, north) values of field b at the row's point 4 tt + i (digit-reversed order).  L is 0 for
 // a row past the last radius.
@@ -238,7 +250,7 @@ __device__ __forceinline__ void pair_c2r(const PhysParams& P, const double* __re
     __syncthreads();
     if constexpr (S::R1 > 1) {
         pair_mid_pass<M, NB, S::R1, Q, false>(buf, P.twq, tt);
-        __syncthreads();
+        mid_barrier<M>(tt);
     }
     pair_mid_pass<M, NB, S::R2, 4 * S::R2, false>(buf, P.twq + S::TW2, tt);
     __syncthreads();
