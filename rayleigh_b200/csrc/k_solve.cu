@@ -333,13 +333,11 @@ __global__ void __launch_bounds__(256) lu_offdiag_kernel(double* __restrict__ ma
 // One CTA per (system, l, NC right-hand-side columns), 8 warps.  The CTA's
 // columns (P b) sit in shared memory for both sweeps.  For block row i the
 // product over its K range is split between two warp groups (K chunks of 16
-// dealt alternately); warp w owns rows 16 (w mod 4) .. +16 of the block row and
+// dealt alternately); warp w owns rows 16 (w / 2) .. +16 of the block row and
 // all NC columns (2 x NC/8 tensor-core tiles, 2 NC/8 x 2 mma per k-step).  Each
 // element of M is used by one warp only, so that the warp streams ITS OWN rows
-// straight into fragment registers, two chunks ahead (a lane takes two
-// neighbouring k of a row with one 16-byte load; the k of an 8-wide group are
-// dealt to two k-steps accordingly), and no CTA-wide barrier is needed until the
-// block row ends: the second group then hands its partial sums to the first
+// straight into fragment registers, two chunks ahead, and no CTA-wide barrier is
+// needed until the block row ends: the second group then hands its partial sums to the first
 // through shared memory, which writes the block row's result over its
 // right-hand side.
 // What bounds it: on small systems the chain of one CTA (load the columns, 2 nblk
@@ -348,7 +346,7 @@ __global__ void __launch_bounds__(256) lu_offdiag_kernel(double* __restrict__ ma
 // after the other took longer than the substitution below n ~ 200), and every
 // system of the step goes out as one launch where two CTAs fit an SM (n <= 384).
 // Without a shared-memory ring for M the block takes 65 KB at n = 144 (three CTAs
-// per SM instead of one) and 98 KB at n = 288 (two).
+// per SM instead of one) and 114 KB at n = 384 (two).
 constexpr int LS_KC = 16;                 // K per chunk
 constexpr int LS_WARPS = 8, LS_THREADS = 32 * LS_WARPS;
 
@@ -365,19 +363,19 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 }
 
 // The column block in shared memory, [row][NC] with the columns of row i
-// permuted by XOR with h(i) = 8 i_1 + (i_0 + 2 i_2 + 4 i_3) (bits of i): a B
-// fragment (rows k + 2 tig, k = 0 mod 8, 8 columns) and a walk down 32
+// permuted by XOR with h(i) = 8 (i mod 2) + (i/2 mod 8): over a warp, a B
+// fragment (rows k..k+3, k = 0 mod 4, 8 columns) and a walk down 32
 // consecutive rows of one column both touch every 8-byte bank exactly twice.
 template <int NC>
 __device__ __forceinline__ int xs_index(int i, int c) {
-    return i * NC + (c ^ (((i & 2) << 2) | (i & 1) | ((i >> 1) & 6)));
+    return i * NC + (c ^ (((i & 1) << 3) | ((i >> 1) & 7)));
 }
 
 template <int NC>
 struct LuSolveShape {
     static size_t smem(int n) {
         const int nrow = (n + SB - 1) / SB * SB;
-        return ((size_t)nrow * NC + (size_t)SB * NC) * sizeof(double) + (size_t)nrow * sizeof(int);
+        return ((size_t)nrow * NC + (size_t)SB * NC) * sizeof(double);
     }
 };
 
@@ -392,7 +390,7 @@ __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4
     const int nblk = (n + SB - 1) / SB, nrow = nblk * SB;
     double* Xs = ssm;                                      // [nrow][NC]
     double* red = Xs + (size_t)nrow * NC;                  // [SB][NC] second group's partial sums
-    int* inv = reinterpret_cast<int*>(red + SB * NC);      // [n] the row a right-hand-side entry goes to
+    int* inv = reinterpret_cast<int*>(red);                // [n] the row a right-hand-side entry goes to (load only)
     const double* __restrict__ M = S.M + (size_t)l * n * n;
     const int* __restrict__ perm = S.perm + (size_t)l * n;
     const double* rhs = nullptr;
@@ -414,25 +412,24 @@ __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4
     const int t = threadIdx.x;
     const int lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, tig = lane & 3;
-    const int rgp = warp & 3, grp = warp >> 2;             // row group (16 rows), K group
+    const int rgp = warp >> 1, grp = warp & 1;             // row group (16 rows), K group
     // this warp's chunks in order over both sweeps: (block row q-th, chunk j = grp, grp + 2, ...);
     // forward block ib has 4 (ib + 1) chunks from k = 0 on; backward block ib has 4 (nblk - ib) from
     // its own first row on
     auto nchunks = [&](bool bw, int ib) { return bw ? 4 * (nblk - ib) : 4 * (ib + 1); };
     int f_bw = 0, f_q = 0, f_j = grp;                      // fetch cursor: sweep, block row ordinal, chunk
-    auto fetch = [&](double2 (&a)[2][2]) {                 // rows g, g + 8 of the warp's 16; k = 8 h + 2 tig + {0, 1}
+    auto fetch = [&](double (&a)[2][4]) {                  // rows g, g + 8 of the warp's 16; k = 4 s + tig
         if (f_bw < 2) {
             const bool bw = f_bw == 1;
             const int ib = bw ? nblk - 1 - f_q : f_q;
-            const int gk0 = (bw ? ib * SB : 0) + f_j * LS_KC + 2 * tig;
+            const int gk0 = (bw ? ib * SB : 0) + f_j * LS_KC + tig;
 #pragma unroll
             for (int mi = 0; mi < 2; ++mi) {
                 const int gr = ib * SB + rgp * 16 + mi * 8 + g;
                 const double* row = M + (size_t)gr * n;
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    a[mi][h] = (gr < n && gk0 + 8 * h < n) ? __ldg(reinterpret_cast<const double2*>(row + gk0 + 8 * h))
-                                                           : make_double2(0.0, 0.0);
+                for (int s = 0; s < 4; ++s)
+                    a[mi][s] = (gr < n && gk0 + 4 * s < n) ? __ldg(row + gk0 + 4 * s) : 0.0;
             }
             f_j += 2;
             if (f_j >= nchunks(bw, ib)) {
@@ -444,7 +441,7 @@ __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4
             }
         }
     };
-    double2 a0[2][2] = {}, a1[2][2] = {};
+    double a0[2][4] = {}, a1[2][4] = {};
     fetch(a0);
     fetch(a1);
     // permuted right-hand sides (P b), zero past n and past the last column; the entries of a column are
@@ -482,34 +479,31 @@ __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4
             for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
                 for (int ni = 0; ni < NT; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0.0;
-            auto multiply = [&](double2 (&a)[2][2], int j) {
+            auto multiply = [&](double (&a)[2][4], int j) {
                 const int k0 = kb + j * LS_KC;
                 if (k0 >= ib * SB && k0 < ib * SB + SB) {   // the diagonal block: L^-1 (unit) or U^-1
+                    const int jd = (k0 - ib * SB) / LS_KC;  // zero above or below the warp's 16 x 16 diagonal chunk
+                    if (bw ? jd < rgp : jd > rgp) return;
 #pragma unroll
                     for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const int rg = ib * SB + rgp * 16 + mi * 8 + g, kg = k0 + 8 * h + 2 * tig;
-                            double2& v = a[mi][h];
-                            v.x = bw ? (kg >= rg ? v.x : 0.0) : (kg < rg ? v.x : (kg == rg ? 1.0 : 0.0));
-                            v.y = bw ? (kg + 1 >= rg ? v.y : 0.0) : (kg + 1 < rg ? v.y : (kg + 1 == rg ? 1.0 : 0.0));
+                        for (int s = 0; s < 4; ++s) {
+                            const int rg = ib * SB + rgp * 16 + mi * 8 + g, kg = k0 + 4 * s + tig;
+                            double& v = a[mi][s];
+                            v = bw ? (kg >= rg ? v : 0.0) : (kg < rg ? v : (kg == rg ? 1.0 : 0.0));
                         }
                 }
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                for (int s = 0; s < 4; ++s) {
+                    const int kg = k0 + 4 * s + tig;
+                    double b[NT];
 #pragma unroll
-                    for (int s = 0; s < 2; ++s) {
-                        const int kg = k0 + 8 * h + 2 * tig + s;
-                        double b[NT];
+                    for (int ni = 0; ni < NT; ++ni) b[ni] = Xs[xs_index<NC>(kg, ni * 8 + g)];
 #pragma unroll
-                        for (int ni = 0; ni < NT; ++ni) b[ni] = Xs[xs_index<NC>(kg, ni * 8 + g)];
+                    for (int mi = 0; mi < 2; ++mi)
 #pragma unroll
-                        for (int mi = 0; mi < 2; ++mi) {
-                            const double av = s ? a[mi][h].y : a[mi][h].x;
-#pragma unroll
-                            for (int ni = 0; ni < NT; ++ni) dmma884(acc[mi][ni], av, b[ni]);
-                        }
-                    }
+                        for (int ni = 0; ni < NT; ++ni) dmma884(acc[mi][ni], a[mi][s], b[ni]);
+                }
             };
             for (int j = grp; j < nch; j += 4) {   // an even number of chunks per group
                 multiply(a0, j);
@@ -788,6 +782,11 @@ static T* upload_vec(Ctx& c, const std::vector<T>& v) {
 void solve_prepare(Ctx& c) {
     c.solve_nc = lu_nc_for(3 * c.d.nr);
     c.solve_nc_z = lu_nc_for(c.d.nr);
+    // Fewer tiles than SMs: narrower ones fill more of them, and a CTA's chain of products halves
+    // (l_max 41, N_r 48: 33 -> 25 us; at l_max 63, 160 tiles, 48 -> 51 us, at 127 138 -> 167 us).
+    long tiles = 0;
+    for (int l = 0; l < c.d.L; ++l) tiles += (2 * (l + 1) + 31) / 32;
+    if (tiles <= 148) c.solve_nc = c.solve_nc_z = 16;
     rebuild_solve_tiles(c);
 }
 
