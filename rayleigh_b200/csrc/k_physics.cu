@@ -121,7 +121,11 @@ __host__ __device__ constexpr int fstride(int n) { return n + 2; }
 
 // One CTA = one (theta, r) row; the rows theta and pi - theta of a pair form a
 // 2-CTA cluster that folds its spectra through distributed shared memory.
-constexpr int ROW_THREADS = 384;
+// Threads of a row CTA: half a thread per complex point, whole warps, at most 384.  The diagnostics
+// transform one or a few fields at a time, N / 8 butterflies a pass: with 384 threads at every N most
+// of them waited at the barriers of a small row, and few rows fitted an SM (n_theta = 192, N_r = 64:
+// shell averages of seven quantities 6.5 -> 2.2 ms, azimuthal 3.5 -> 1.4, global 3.4 -> 1.3).
+__host__ __device__ constexpr int row_threads(int n) { return n >= 768 ? 384 : (n / 2 + 31) / 32 * 32; }
 constexpr int FB = 4;   // fields per batched FFT
 
 // Shared memory of a row CTA (double2 units): one in-place FFT buffer of FB
@@ -320,14 +324,14 @@ __device__ __forceinline__ T pick(const T (&a)[NB], int b) {
 // c2r of NB fields of this row (fields fo[b], d/dphi where dp[b]; mpart as in spec_value,
 // 0 in the time step): the input Z is formed straight from the spectrum loads (one (k, N-k)
 // pair per work item), then the DIF passes.  On return y[b][q] holds the physical pair
-// (y[2n], y[2n+1]) of field b at the buffer position t + q*ROW_THREADS.
+// (y[2n], y[2n+1]) of field b at the buffer position t + q*row_threads(N).
 template <int N, int NB, int ZPT>
 __device__ __forceinline__ void row_c2r(const PhysParams& P, const double* __restrict__ rowbase, int h,
                                         const int (&fo)[NB], const bool (&dp)[NB], double2* sm, int t,
                                         double2 (&y)[FB][ZPT], int mpart = 0) {
     constexpr int FS = fstride(N);
     constexpr int NI = N / 2 + 1;                                   // k = 0 .. N/2
-    constexpr int QI = (NB * NI + ROW_THREADS - 1) / ROW_THREADS;   // items per thread
+    constexpr int QI = (NB * NI + row_threads(N) - 1) / row_threads(N);   // items per thread
     double2* buf = sm + RowSmem<N>::BUF;
     const int L = P.L;
     const long ostride = (long)P.ncola;   // E -> O within p2a[theta_h][m][par][r][field][2]
@@ -353,7 +357,7 @@ __device__ __forceinline__ void row_c2r(const PhysParams& P, const double* __res
         double2 xk[QC], xn[QC];
 #pragma unroll
         for (int qq = 0; qq < QC; ++qq) {
-            const int g = t + (q0 + qq) * ROW_THREADS;
+            const int g = t + (q0 + qq) * row_threads(N);
             xk[qq] = xn[qq] = make_double2(0.0, 0.0);
             if (q0 + qq < QI && g < NB * NI) {
                 int k, b;
@@ -366,7 +370,7 @@ __device__ __forceinline__ void row_c2r(const PhysParams& P, const double* __res
         }
 #pragma unroll
         for (int qq = 0; qq < QC; ++qq) {
-            const int g = t + (q0 + qq) * ROW_THREADS;
+            const int g = t + (q0 + qq) * row_threads(N);
             if (q0 + qq < QI && g < NB * NI) {
                 int k, b;
                 item(g, k, b);
@@ -377,12 +381,12 @@ __device__ __forceinline__ void row_c2r(const PhysParams& P, const double* __res
         }
     }
     __syncthreads();
-    fft_dif<N, NB, ROW_THREADS>(buf, P.twp, t);
+    fft_dif<N, NB, row_threads(N)>(buf, P.twp, t);
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
         for (int q = 0; q < ZPT; ++q) {
-            const int n = t + q * ROW_THREADS;
+            const int n = t + q * row_threads(N);
             y[b][q] = (n < N) ? buf[SW(b * FS + n)] : make_double2(0.0, 0.0);
         }
 }
@@ -395,7 +399,7 @@ __device__ __forceinline__ void r2c_finish(double2* a, int nf, int L, const doub
                                            const HS& hsf) {
     constexpr int FS = fstride(N);
     constexpr int NI = N / 2 + 1;
-    for (int g = t; g < nf * NI; g += ROW_THREADS) {
+    for (int g = t; g < nf * NI; g += row_threads(N)) {
         const int f = g / NI, k = g - f * NI;
         const double2 zk = a[SW(f * FS + k)];
         const double2 zn = a[SW(f * FS + (N - k) % N)];
@@ -882,13 +886,13 @@ void launch_fft_rows(Ctx& c, double* d_x, long howmany, int inverse) {
 // integration weights (Compute_Radial_Average).  No cluster: each row reads
 // its own hemisphere's reflection of the even and odd parts.
 template <int N, bool ME>
-__global__ void __launch_bounds__(ROW_THREADS) kinetic_energy_rows_kernel(PhysParams P, const double* __restrict__ kew,
+__global__ void __launch_bounds__(row_threads(N)) kinetic_energy_rows_kernel(PhysParams P, const double* __restrict__ kew,
                                                                           double* __restrict__ rows) {
     // ME: |B|^2 from B_r and r sin(theta) B_theta, B_phi (Benchmarking.F90:689-696), else rho |u|^2 / 2
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* sm = reinterpret_cast<double2*>(smem_raw);
-    __shared__ double red[ROW_THREADS / 32];
+    __shared__ double red[row_threads(N) / 32];
     const int t = threadIdx.x;
     const int h = (int)(blockIdx.x & 1);
     const int nr = P.nr;
@@ -910,7 +914,7 @@ __global__ void __launch_bounds__(ROW_THREADS) kinetic_energy_rows_kernel(PhysPa
     double s = 0.0;
 #pragma unroll
     for (int q = 0; q < ZPT; ++q)
-        if (t + q * ROW_THREADS < N) {
+        if (t + q * row_threads(N) < N) {
             const double2 a = y[0][q];
             const double2 b = make_double2(y[1][q].x * csc, y[1][q].y * csc);
             const double2 c = make_double2(y[2][q].x * csc, y[2][q].y * csc);
@@ -921,7 +925,7 @@ __global__ void __launch_bounds__(ROW_THREADS) kinetic_energy_rows_kernel(PhysPa
     __syncthreads();
     if (t == 0) {
         double v = red[0];
-        for (int i = 1; i < ROW_THREADS / 32; ++i) v += red[i];
+        for (int i = 1; i < row_threads(N) / 32; ++i) v += red[i];
         const double w = ME ? 1.0 : 0.5 * P.radial[R_DENSITY * nr + r];
         rows[(long)th * nr + r] = w * v * kew[th] * kew[N + r];
     }
@@ -964,7 +968,7 @@ void launch_kinetic_energy(Ctx& c, bool magnetic) {
     auto go = [&](auto kern, int n) {
         const size_t smem = (size_t)3 * fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P, c.d_kew, c.d_ke_rows);
+        kern<<<grid, row_threads(n), smem, c.stream>>>(P, c.d_kew, c.d_ke_rows);
     };
     switch (c.d.nth) {
         case 24: if (magnetic) go(kinetic_energy_rows_kernel<24, true>, 24); else go(kinetic_energy_rows_kernel<24, false>, 24); break;
@@ -1081,8 +1085,8 @@ __device__ __forceinline__ double row_quantity(const PhysParams& P, const SliceS
 // physical-space stage divides by it) and writes the row in natural phi order:
 // out[level][theta][phi].
 template <int N>
-__global__ void __launch_bounds__(ROW_THREADS) shell_slice_kernel(PhysParams P, SliceSpec S, double* __restrict__ out) {
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+__global__ void __launch_bounds__(row_threads(N)) shell_slice_kernel(PhysParams P, SliceSpec S, double* __restrict__ out) {
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* sm = reinterpret_cast<double2*>(smem_raw);
     const int t = threadIdx.x;
@@ -1097,7 +1101,7 @@ __global__ void __launch_bounds__(ROW_THREADS) shell_slice_kernel(PhysParams P, 
     double2* row = reinterpret_cast<double2*>(out + ((long)lv * N + th) * (2L * N));
 #pragma unroll
     for (int q = 0; q < ZPT; ++q) {
-        const int p = t + q * ROW_THREADS;
+        const int p = t + q * row_threads(N);
         if (p < N) row[natural_index<N>(p)] = make_double2(y[0][q].x * scale, y[0][q].y * scale);
     }
 }
@@ -1121,7 +1125,7 @@ void launch_shell_slice(Ctx& c, const SliceSpec& S, double* out) {
     auto go = [&](auto kern, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, out);
+        kern<<<grid, row_threads(n), smem, c.stream>>>(P, S, out);
     };
     switch (c.d.nth) {
         case 24: go(shell_slice_kernel<24>, 24); break;
@@ -1148,14 +1152,14 @@ void launch_shell_slice(Ctx& c, const SliceSpec& S, double* out) {
 // of (q - mean(r))^m for m = 2, 3, 4 (slots 1-3).  rows[slot][theta][r];
 // kew[theta] = Gauss-Legendre weight / 2 / n_phi.
 template <int N, bool MOMENTS>
-__global__ void __launch_bounds__(ROW_THREADS) shell_moment_rows_kernel(PhysParams P, SliceSpec S,
+__global__ void __launch_bounds__(row_threads(N)) shell_moment_rows_kernel(PhysParams P, SliceSpec S,
                                                                         const double* __restrict__ kew,
                                                                         const double* __restrict__ mean,
                                                                         double* __restrict__ rows) {
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* sm = reinterpret_cast<double2*>(smem_raw);
-    __shared__ double red[3][ROW_THREADS / 32];
+    __shared__ double red[3][row_threads(N) / 32];
     const int t = threadIdx.x;
     const int h = (int)(blockIdx.x & 1);
     const int thh = (int)(blockIdx.x >> 1);
@@ -1169,7 +1173,7 @@ __global__ void __launch_bounds__(ROW_THREADS) shell_moment_rows_kernel(PhysPara
     double s1 = 0.0, s2 = 0.0, s3 = 0.0;
 #pragma unroll
     for (int q = 0; q < ZPT; ++q)
-        if (t + q * ROW_THREADS < N) {
+        if (t + q * row_threads(N) < N) {
             const double a = y[0][q].x * scale - mu, b = y[0][q].y * scale - mu;
             if (MOMENTS) {
                 const double a2 = a * a, b2 = b * b;
@@ -1195,7 +1199,7 @@ __global__ void __launch_bounds__(ROW_THREADS) shell_moment_rows_kernel(PhysPara
     __syncthreads();
     if (t < (MOMENTS ? 3 : 1)) {
         double v = red[t][0];
-        for (int i = 1; i < ROW_THREADS / 32; ++i) v += red[t][i];
+        for (int i = 1; i < row_threads(N) / 32; ++i) v += red[t][i];
         const int slot = MOMENTS ? 1 + t : 0;
         rows[((long)slot * N + th) * nr + r] = v * kew[th];
     }
@@ -1240,11 +1244,11 @@ void launch_shell_moments(Ctx& c, const SliceSpec& S, double* rows, double* out)
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         RA_CUDA(cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k0<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, c.d_kew, out, rows);
+        k0<<<grid, row_threads(n), smem, c.stream>>>(P, S, c.d_kew, out, rows);
         RA_CUDA(cudaGetLastError());
         shell_reduce_kernel<<<dim3((unsigned)c.d.nr, 1), 256, 0, c.stream>>>(rows, c.d.nth, c.d.nr, 0, out);
         RA_CUDA(cudaGetLastError());
-        k1<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, c.d_kew, out, rows);   // reads the mean, out[0][r]
+        k1<<<grid, row_threads(n), smem, c.stream>>>(P, S, c.d_kew, out, rows);   // reads the mean, out[0][r]
         RA_CUDA(cudaGetLastError());
         shell_reduce_kernel<<<dim3((unsigned)c.d.nr, 3), 256, 0, c.stream>>>(rows, c.d.nth, c.d.nr, 1, out);
         RA_CUDA(cudaGetLastError());
@@ -1289,7 +1293,7 @@ void launch_azimuthal_average(Ctx& c, const SliceSpec& S, double* rows) {
     auto go = [&](auto k0, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k0<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, c.d_kaz, nullptr, rows);
+        k0<<<grid, row_threads(n), smem, c.stream>>>(P, S, c.d_kaz, nullptr, rows);
     };
 #define RA_AZ(n) go(shell_moment_rows_kernel<n, false>, n)
     switch (c.d.nth) {
@@ -1318,9 +1322,9 @@ void launch_azimuthal_average(Ctx& c, const SliceSpec& S, double* rows) {
 // into the p2b layout at the column slot slot0 + level index; the forward
 // Legendre transform of that buffer then gives the (l, m) coefficients.
 template <int N>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROW_THREADS)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(row_threads(N))
     spectra_rows_kernel(PhysParams P, SliceSpec S, int slot0, double* __restrict__ p2b) {
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     constexpr int NI = N / 2 + 1;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -1337,13 +1341,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROW_THREADS)
     const double scale = row_quantity<N, ZPT>(P, S, rowbase, h, th, r, buf, t, y);
 #pragma unroll
     for (int q = 0; q < ZPT; ++q) {   // each thread rewrites the positions it read
-        const int p = t + q * ROW_THREADS;
+        const int p = t + q * row_threads(N);
         if (p < N) buf[p] = make_double2(y[0][q].x * scale, y[0][q].y * scale);
     }
     __syncthreads();
-    fft_dit<N, 1, ROW_THREADS>(buf, P.twp, t);
+    fft_dit<N, 1, row_threads(N)>(buf, P.twp, t);
     const int L = P.L;
-    for (int k = t; k < NI; k += ROW_THREADS) {   // r2c steps, one (k, N - k) pair per item, in place
+    for (int k = t; k < NI; k += row_threads(N)) {   // r2c steps, one (k, N - k) pair per item, in place
         const double2 zk = buf[k];
         const double2 zn = buf[(N - k) % N];
         const double2 wk = __ldg(P.wr + k);
@@ -1365,7 +1369,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROW_THREADS)
         const long ncolb = (long)P.nfb * P.nr * 2;
         const long mstride = 2L * (N / 2) * ncolb;   // p2b[m][par][theta_h][col]
         double* obase = p2b + (long)h * (N / 2) * ncolb + (long)thh * ncolb + (long)(slot0 + lv) * 2;
-        for (int k = t; k < L; k += ROW_THREADS) {
+        for (int k = t; k < L; k += row_threads(N)) {
             const double2 a = buf[k], b = peer[k];
             *reinterpret_cast<double2*>(obase + k * mstride) = h ? csub(b, a) : cadd(a, b);
         }
@@ -1408,7 +1412,7 @@ void launch_spectra_rows(Ctx& c, const SliceSpec& S, int slot0, double* p2b) {
     auto go = [&](auto kern, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, slot0, p2b);
+        kern<<<grid, row_threads(n), smem, c.stream>>>(P, S, slot0, p2b);
     };
     switch (c.d.nth) {
         case 24: go(spectra_rows_kernel<24>, 24); break;
@@ -1442,9 +1446,9 @@ void launch_spectra_gather(Ctx& c, const double* s2, int nslots, double* out) {
 // shell_slice_kernel) and rank 0 averages the two through distributed shared
 // memory into out[r][phi] (natural phi order).  One cluster per radius.
 template <int N>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROW_THREADS)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(row_threads(N))
     equatorial_slice_kernel(PhysParams P, SliceSpec S, double* __restrict__ out) {
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1459,14 +1463,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(ROW_THREADS)
     const double scale = row_quantity<N, ZPT>(P, S, rowbase, h, th, r, buf, t, y);
 #pragma unroll
     for (int q = 0; q < ZPT; ++q) {   // each thread rewrites the positions it read
-        const int p = t + q * ROW_THREADS;
+        const int p = t + q * row_threads(N);
         if (p < N) buf[p] = make_double2(y[0][q].x * scale, y[0][q].y * scale);
     }
     cluster.sync();
     if (h == 0) {
         const double2* peer = cluster.map_shared_rank(buf, 1);
         double2* row = reinterpret_cast<double2*>(out + (long)r * (2L * N));
-        for (int p = t; p < N; p += ROW_THREADS) {
+        for (int p = t; p < N; p += row_threads(N)) {
             const double2 a = buf[p], b = peer[p];
             row[natural_index<N>(p)] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
         }
@@ -1492,7 +1496,7 @@ void launch_equatorial_slice(Ctx& c, const SliceSpec& S, double* out) {
     auto go = [&](auto kern, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, out);
+        kern<<<grid, row_threads(n), smem, c.stream>>>(P, S, out);
     };
     switch (c.d.nth) {
         case 24: go(equatorial_slice_kernel<24>, 24); break;
@@ -1517,9 +1521,9 @@ void launch_equatorial_slice(Ctx& c, const SliceSpec& S, double* out) {
 // one CTA per row forms the row on the phi grid, puts it in natural order in
 // shared memory and writes the chosen points to out[j][theta][r].
 template <int N>
-__global__ void __launch_bounds__(ROW_THREADS) meridional_slice_kernel(PhysParams P, SliceSpec S,
+__global__ void __launch_bounds__(row_threads(N)) meridional_slice_kernel(PhysParams P, SliceSpec S,
                                                                        double* __restrict__ out) {
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* buf = reinterpret_cast<double2*>(smem_raw);
     const int t = threadIdx.x;
@@ -1534,12 +1538,12 @@ __global__ void __launch_bounds__(ROW_THREADS) meridional_slice_kernel(PhysParam
     __syncthreads();   // every thread has read its points out of the buffer
 #pragma unroll
     for (int q = 0; q < ZPT; ++q) {
-        const int p = t + q * ROW_THREADS;
+        const int p = t + q * row_threads(N);
         if (p < N) buf[natural_index<N>(p)] = make_double2(y[0][q].x * scale, y[0][q].y * scale);
     }
     __syncthreads();
     const double* row = reinterpret_cast<const double*>(buf);   // natural phi order
-    for (int j = t; j < S.nl; j += ROW_THREADS) out[((long)j * N + th) * nr + r] = row[S.level[j]];
+    for (int j = t; j < S.nl; j += row_threads(N)) out[((long)j * N + th) * nr + r] = row[S.level[j]];
 }
 
 void launch_meridional_slice(Ctx& c, const SliceSpec& S, double* out) {
@@ -1561,7 +1565,7 @@ void launch_meridional_slice(Ctx& c, const SliceSpec& S, double* out) {
     auto go = [&](auto kern, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, out);
+        kern<<<grid, row_threads(n), smem, c.stream>>>(P, S, out);
     };
     switch (c.d.nth) {
         case 24: go(meridional_slice_kernel<24>, 24); break;
@@ -1612,7 +1616,7 @@ void launch_global_average(Ctx& c, const SliceSpec& S, double* rows, double* mea
     auto go = [&](auto k0, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k0<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, c.d_kew, nullptr, rows);
+        k0<<<grid, row_threads(n), smem, c.stream>>>(P, S, c.d_kew, nullptr, rows);
     };
 #define RA_GA(n) go(shell_moment_rows_kernel<n, false>, n)
     switch (c.d.nth) {
@@ -1643,9 +1647,9 @@ void launch_global_average(Ctx& c, const SliceSpec& S, double* rows, double* mea
 // grid, in natural order in shared memory, and writes the chosen phi points to
 // out[r_i][theta_j][phi_k].
 template <int N>
-__global__ void __launch_bounds__(ROW_THREADS) point_probe_kernel(PhysParams P, SliceSpec S, ProbeSet Q,
+__global__ void __launch_bounds__(row_threads(N)) point_probe_kernel(PhysParams P, SliceSpec S, ProbeSet Q,
                                                                   double* __restrict__ out) {
-    constexpr int ZPT = (N + ROW_THREADS - 1) / ROW_THREADS;
+    constexpr int ZPT = (N + row_threads(N) - 1) / row_threads(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2* buf = reinterpret_cast<double2*>(smem_raw);
     const int t = threadIdx.x;
@@ -1659,12 +1663,12 @@ __global__ void __launch_bounds__(ROW_THREADS) point_probe_kernel(PhysParams P, 
     __syncthreads();   // every thread has read its points out of the buffer
 #pragma unroll
     for (int q = 0; q < ZPT; ++q) {
-        const int p = t + q * ROW_THREADS;
+        const int p = t + q * row_threads(N);
         if (p < N) buf[natural_index<N>(p)] = make_double2(y[0][q].x * scale, y[0][q].y * scale);
     }
     __syncthreads();
     const double* row = reinterpret_cast<const double*>(buf);
-    for (int k = t; k < Q.nphi; k += ROW_THREADS)
+    for (int k = t; k < Q.nphi; k += row_threads(N))
         out[((long)ir * Q.ntheta + jt) * Q.nphi + k] = row[Q.phi[k]];
 }
 
@@ -1686,7 +1690,7 @@ void launch_point_probes(Ctx& c, const SliceSpec& S, const ProbeSet& Q, double* 
     auto go = [&](auto kern, int n) {
         const size_t smem = (size_t)fstride(n) * sizeof(double2);
         RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<grid, ROW_THREADS, smem, c.stream>>>(P, S, Q, out);
+        kern<<<grid, row_threads(n), smem, c.stream>>>(P, S, Q, out);
     };
     switch (c.d.nth) {
         case 24: go(point_probe_kernel<24>, 24); break;
