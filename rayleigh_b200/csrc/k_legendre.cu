@@ -13,7 +13,7 @@
 //  All m share one launch; K (the number of l of one parity) is ragged and the
 //  grid is ordered by m so that the long products start first.
 #include "ra_internal.h"
-#include "gemm_async.cuh"
+#include "gemm_f64.cuh"
 
 namespace ra {
 
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 4) lt_inverse_kernel(const doubl
     const long roff = m_off(m, L) + (par ? ne : 0);
     Acc acc;
     acc.zero();
-    gemm_async<false>(acc, OA{Ptab + roff * nth2 + th0, nth2, nl, nth2 - th0}, OB{s2 + roff * ncol + c0, ncol, nl, ncol - c0},
+    gemm_async<false, false>(acc, OA{Ptab + roff * nth2 + th0, nth2, nl, nth2 - th0}, OB{s2 + roff * ncol + c0, ncol, nl, ncol - c0},
                       nl, ga_sm);
     double* out = p2 + (long)blockIdx.z * ncol + c0;
     const long th_stride = 2L * L * ncol;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 4) lt_forward_kernel(const doubl
     const long roff = m_off(m, L) + (par ? ne : 0) + l0;
     Acc acc;
     acc.zero();
-    gemm_async<true>(acc, FwdA{iPtab + roff * nth2, nth2, nth2, nl - l0},
+    gemm_async<true, false>(acc, FwdA{iPtab + roff * nth2, nth2, nth2, nl - l0},
                      FwdB{p2 + ((long)m * 2 + par) * nth2 * ncol + c0, ncol, nth2, ncol - c0}, nth2, ga_sm);
     double* out = s2 + roff * ncol + c0;
     acc_each<true>(acc, [&](int x, int y, double v0, double v1) {

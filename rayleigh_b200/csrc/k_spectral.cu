@@ -270,7 +270,7 @@ static_assert(slot_eq(3) == kSlots[3].eq && slot_g(8) == kSlots[8].g && slot_g(1
 
 // w2s (finite-difference mode only, else NULL): the plane of d/dr (dW/dr) that Post_Solve_FD's
 // deriv_cluge sends on to rlm_spacea in place of d2W/dr2 (Sphere_Spectral_Space.F90:96-98).
-__global__ void post_assemble_kernel(const double* __restrict__ g, const double* __restrict__ ab,
+__device__ __forceinline__ void post_assemble_part(const double* __restrict__ g, const double* __restrict__ ab,
                                      const double* __restrict__ coef, double* __restrict__ rhs_wpt,
                                      double* __restrict__ rhs_z, double* __restrict__ s2a, long nlm, int nr,
                                      int L, double old_ab, const double* __restrict__ w2s) {
@@ -321,18 +321,9 @@ __global__ void post_assemble_kernel(const double* __restrict__ g, const double*
     *reinterpret_cast<double2*>(o + (NS2A - 1) * fs) = w2;
 }
 
-void launch_post_assemble(Ctx& c, double old_ab) {
-    const long total = c.d.nlm * c.d.nr;
-    const double* w2s = c.cfg.chebyshev ? nullptr : c.d_g + (size_t)c.ng * c.d.nlm * 2 * c.d.nr;
-    post_assemble_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c.stream>>>(
-        c.d_g, c.d_ab, c.d_coef, c.d_rhs_wpt, c.d_rhs_z, c.d_s2a, c.d.nlm, c.d.nr, c.d.L, old_ab, w2s);
-    RA_CUDA(cudaGetLastError());
-    ++c.launches;
-}
-
 // The C and A parts of Post_Solve (Sphere_Spectral_Space.F90:268-297, 370-384): their
 // right-hand sides, and the fields rlm_spacea's magnetic part reads, m-major.
-__global__ void post_assemble_mag_kernel(const double* __restrict__ g, const double* __restrict__ ab,
+__device__ __forceinline__ void post_assemble_mag_part(const double* __restrict__ g, const double* __restrict__ ab,
                                          const double* __restrict__ coefm, double* __restrict__ rhs_c,
                                          double* __restrict__ rhs_a, double* __restrict__ s2am, long nlm, int nr,
                                          int L, double old_ab) {
@@ -377,10 +368,27 @@ __global__ void post_assemble_mag_kernel(const double* __restrict__ g, const dou
         *reinterpret_cast<double2*>(so + f * fs) = make_double2(gv[kOut[f] - G_C0][0], gv[kOut[f] - G_C0][1]);
 }
 
-void launch_post_assemble_mag(Ctx& c, double old_ab) {
+// With magnetism the C and A parts are the second half of the launch's grid (y = 1): on a small grid
+// the two halves run side by side.
+__global__ void post_assemble_kernel(const double* __restrict__ g, const double* __restrict__ ab,
+                                     const double* __restrict__ coef, const double* __restrict__ coefm,
+                                     double* __restrict__ rhs_wpt, double* __restrict__ rhs_z,
+                                     double* __restrict__ rhs_c, double* __restrict__ rhs_a, double* __restrict__ s2a,
+                                     double* __restrict__ s2am, long nlm, int nr, int L, double old_ab,
+                                     const double* __restrict__ w2s) {
+    if (blockIdx.y == 0)
+        post_assemble_part(g, ab, coef, rhs_wpt, rhs_z, s2a, nlm, nr, L, old_ab, w2s);
+    else
+        post_assemble_mag_part(g, ab, coefm, rhs_c, rhs_a, s2am, nlm, nr, L, old_ab);
+}
+
+void launch_post_assemble(Ctx& c, double old_ab) {
     const long total = c.d.nlm * c.d.nr;
-    post_assemble_mag_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c.stream>>>(
-        c.d_g, c.d_ab, c.d_coef_mag, c.d_rhs_c, c.d_rhs_a, c.d_s2am, c.d.nlm, c.d.nr, c.d.L, old_ab);
+    const double* w2s = c.cfg.chebyshev ? nullptr : c.d_g + (size_t)c.ng * c.d.nlm * 2 * c.d.nr;
+    const dim3 grid((unsigned)((total + 255) / 256), c.mag ? 2 : 1);
+    post_assemble_kernel<<<grid, 256, 0, c.stream>>>(c.d_g, c.d_ab, c.d_coef, c.d_coef_mag, c.d_rhs_wpt, c.d_rhs_z,
+                                                     c.d_rhs_c, c.d_rhs_a, c.d_s2a, c.d_s2am, c.d.nlm, c.d.nr, c.d.L,
+                                                     old_ab, w2s);
     RA_CUDA(cudaGetLastError());
     ++c.launches;
 }
@@ -588,9 +596,18 @@ void launch_rlm_a(Ctx& c) {
 // ---------------------------------------------------------------------------
 // rlm_spaceb: curl algebra on the transformed NL terms, written l-major (p1b)
 // ---------------------------------------------------------------------------
+// MAG: Adjust_Emf (Sphere_Hybrid_Space.F90:557-602) and the first half of Finalize_EMF in the same
+// thread, so that the records of s2b, whose seven fields share sectors, are read once: the C
+// right-hand side from the radial curl of the EMF,
+//   N_C = (sd_theta EMF_phi - d_phi EMF_theta) / l(l+1),
+// the A one's EMF_r part, and X = (d_phi EMF_phi + sd_theta EMF_theta) / l(l+1), whose
+// radial derivative emf_radial_kernel adds (1 / l(l+1) -> 1 at l = 0, l_max zeroed).
+// Then AB history, Add_To_All_RHS and the (zero) magnetic boundary rows for C.
+template <bool MAG>
 __global__ void rlm_b_kernel(const double* __restrict__ s2b, double* __restrict__ ab, double* __restrict__ rhs_wpt,
-                             double* __restrict__ rhs_z, long nlm, int nr, int L, double new_ab, double bc_top,
-                             double bc_bot, const double* __restrict__ bcv, int* __restrict__ status, int nfb) {
+                             double* __restrict__ rhs_z, double* __restrict__ rhs_c, double* __restrict__ xemf,
+                             long nlm, int nr, int L, double new_ab, double bc_top, double bc_bot,
+                             const double* __restrict__ bcv, int* __restrict__ status, int nfb) {
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;   // (lm, r)
     if (idx >= nlm * nr) return;
     const int r = (int)(idx % nr);
@@ -668,6 +685,27 @@ __global__ void rlm_b_kernel(const double* __restrict__ s2b, double* __restrict_
             rhs_z[o] += new_ab * Z;
         }
     }
+    if constexpr (MAG) {
+        const double2 et = get2(B_EMFT, l), er = get2(B_EMFR, l), ep = get2(B_EMFP, l);
+        const double2 etm = get2(B_EMFT, l - 1), etp = get2(B_EMFT, l + 1);
+        const double2 epm = get2(B_EMFP, l - 1), epp = get2(B_EMFP, l + 1);
+        auto c = [](double2 v, int ri) { return ri ? v.y : v.x; };
+#pragma unroll
+        for (int ri = 0; ri < 2; ++ri) {
+            const double sg = ri ? (double)m : -(double)m;
+            const int rj = 1 - ri;
+            double nc = ((c(epm, ri) * c1 + c(epp, ri) * c2) - sg * c(et, rj)) * ollp1;
+            double x = (sg * c(ep, rj) + (c(etm, ri) * c1 + c(etp, ri) * c2)) * ollp1;
+            double na = c(er, ri);
+            if (l == lmax) nc = x = na = 0.0;
+            if (!(isfinite(nc) && isfinite(x) && isfinite(na))) atomicOr(status, RA_STATUS_NONFINITE);
+            const long o = (lm * 2 + ri) * nr + r;
+            ab[4 * plane + o] = nc;
+            ab[5 * plane + o] = na;   // emf_radial_kernel adds d/dr X
+            xemf[o] = x;
+            rhs_c[o] = edge ? 0.0 : rhs_c[o] + new_ab * nc;
+        }
+    }
 }
 
 static void bc_values(const Ctx& c, double& top, double& bot) {
@@ -710,92 +748,64 @@ void launch_rlm_b(Ctx& c, double new_ab) {
     const long total = c.d.nlm * c.d.nr;
     double top, bot;
     bc_values(c, top, bot);
-    rlm_b_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c.stream>>>(c.d_s2b, c.d_ab, c.d_rhs_wpt, c.d_rhs_z,
-                                                                        c.d.nlm, c.d.nr, c.d.L, new_ab, top, bot,
-                                                                        c.d_bcval, c.d_status, c.nfb);
+    auto go = [&](auto kern) {
+        kern<<<(unsigned)((total + 255) / 256), 256, 0, c.stream>>>(c.d_s2b, c.d_ab, c.d_rhs_wpt, c.d_rhs_z, c.d_rhs_c,
+                                                                    c.d_xemf, c.d.nlm, c.d.nr, c.d.L, new_ab, top, bot,
+                                                                    c.d_bcval, c.d_status, c.nfb);
+    };
+    if (c.mag)
+        go(rlm_b_kernel<true>);
+    else
+        go(rlm_b_kernel<false>);
     RA_CUDA(cudaGetLastError());
     ++c.launches;
-}
-
-// Adjust_Emf (Sphere_Hybrid_Space.F90:557-602) and the first half of Finalize_EMF: the C
-// right-hand side from the radial curl of the EMF,
-//   N_C = (sd_theta EMF_phi - d_phi EMF_theta) / l(l+1),
-// the A one's EMF_r part, and X = (d_phi EMF_phi + sd_theta EMF_theta) / l(l+1), whose
-// radial derivative emf_radial_kernel adds (1 / l(l+1) -> 1 at l = 0, l_max zeroed).
-// Then AB history, Add_To_All_RHS and the (zero) magnetic boundary rows for C.
-__global__ void rlm_b_mag_kernel(const double* __restrict__ s2b, double* __restrict__ ab,
-                                 double* __restrict__ rhs_c, double* __restrict__ xemf, long nlm, int nr, int L,
-                                 double new_ab, int nfb, int* __restrict__ status) {
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;   // (lm, r)
-    if (idx >= nlm * nr) return;
-    const int r = (int)(idx % nr);
-    const long lm = idx / nr;
-    const int l = ell_of_lm(lm);
-    const int m = (int)(lm - (long)l * (l + 1) / 2);
-    const int lmax = L - 1;
-    const long rsz = 2L * nfb * nr;
-    auto get2 = [&](int f, int ll) -> double2 {
-        if (ll < m || ll > lmax) return make_double2(0.0, 0.0);
-        return __ldg(reinterpret_cast<const double2*>(s2b + row_index(m, ll, L) * rsz + r * (2 * nfb) + f * 2));
-    };
-    const double2 et = get2(B_EMFT, l), er = get2(B_EMFR, l), ep = get2(B_EMFP, l);
-    const double2 etm = get2(B_EMFT, l - 1), etp = get2(B_EMFT, l + 1);
-    const double2 epm = get2(B_EMFP, l - 1), epp = get2(B_EMFP, l + 1);
-    auto c = [](double2 v, int ri) { return ri ? v.y : v.x; };
-    const double ollp1 = (l > 0) ? 1.0 / ((double)l * (l + 1)) : 1.0;
-    const double c1 = sdth_c1(l, m), c2 = sdth_c2(l, m);
-    const long plane = nlm * 2 * nr;
-    const bool edge = (r == 0 || r == nr - 1);
-#pragma unroll
-    for (int ri = 0; ri < 2; ++ri) {
-        const double sg = ri ? (double)m : -(double)m;
-        const int rj = 1 - ri;
-        double nc = ((c(epm, ri) * c1 + c(epp, ri) * c2) - sg * c(et, rj)) * ollp1;
-        double x = (sg * c(ep, rj) + (c(etm, ri) * c1 + c(etp, ri) * c2)) * ollp1;
-        double na = c(er, ri);
-        if (l == lmax) nc = x = na = 0.0;
-        if (!(isfinite(nc) && isfinite(x) && isfinite(na))) atomicOr(status, RA_STATUS_NONFINITE);
-        const long o = (lm * 2 + ri) * nr + r;
-        ab[4 * plane + o] = nc;
-        ab[5 * plane + o] = na;   // emf_radial_kernel adds d/dr X
-        xemf[o] = x;
-        rhs_c[o] = edge ? 0.0 : rhs_c[o] + new_ab * nc;
-    }
 }
 
 // Finalize_EMF's radial derivative (Sphere_Spectral_Space.F90:436-488) as one product with
 // the grid operator M (to_spectral, d/dr, dealias, from_spectral): N_A = EMF_r + M X per
 // (l, m, re/im) column, on the FP64 tensor-core tile engine; then the A history, the A
 // right-hand side and its (zero) boundary rows.
-__global__ void __launch_bounds__(GEMM_THREADS, 4) emf_radial_kernel(const double* __restrict__ M,
+__global__ void __launch_bounds__(GEMM_THREADS, 3) emf_radial_kernel(const double* __restrict__ M,
                                                                   const double* __restrict__ xemf,
                                                                   double* __restrict__ ab_a,
                                                                   double* __restrict__ rhs_a, int nr, long ncols,
                                                                   double new_ab) {
-    __shared__ GemmSmem sm;
-    const int r0 = blockIdx.y * Sq::BM;
-    const long c0 = (long)blockIdx.x * Sq::BN;
-    auto fa = [&](int k, int x) -> double {   // M(r0 + x, k)
-        const int rr = r0 + x;
-        return (k < nr && rr < nr) ? __ldg(M + (long)rr * nr + k) : 0.0;
-    };
-    auto fb = [&](int k, int y) -> double {   // X(k, c0 + y)
-        const long col = c0 + y;
-        return (k < nr && col < ncols) ? __ldg(xemf + col * nr + k) : 0.0;
-    };
+    extern __shared__ __align__(16) double ga_sm[];
+    const int r0 = blockIdx.y * GA_BM;
+    const long c0 = (long)blockIdx.x * GA_BN;
     Acc acc;
     acc.zero();
-    gemm_tile<false, false>(acc, fa, fb, nr, sm);
-    acc_foreach(acc, [&](int x, int y, double v) {
-        const int rr = r0 + x;
-        const long col = c0 + y;
-        if (rr < nr && col < ncols) {
-            const long o = col * nr + rr;
-            const double na = ab_a[o] + v;
-            ab_a[o] = na;
-            rhs_a[o] = (rr == 0 || rr == nr - 1) ? 0.0 : rhs_a[o] + new_ab * na;
+    // M(r0 + x, k) and X(k, c0 + y), k contiguous in both
+    gemm_async<true, true>(acc, OperandK{M + (long)r0 * nr, nr, nr, nr - r0},
+                           OperandK{xemf + c0 * nr, nr, nr, (int)min((long)GA_BN, ncols - c0)}, nr, ga_sm);
+    // eight elements at a time: their loads go out together (one element after the other, every load
+    // waited for the store before it)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, tig = lane & 3, wm = warp & 1, wn = warp >> 1;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int rr = r0 + wm * 32 + i * 8 + g;
+        const bool edge = rr == 0 || rr == nr - 1;
+        double a[8], b[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const long col = c0 + wn * 32 + (e >> 1) * 8 + 2 * tig + (e & 1);
+            a[e] = b[e] = 0.0;
+            if (rr < nr && col < ncols) {
+                a[e] = ab_a[col * nr + rr];
+                b[e] = rhs_a[col * nr + rr];
+            }
         }
-    });
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const long col = c0 + wn * 32 + (e >> 1) * 8 + 2 * tig + (e & 1);
+            if (rr < nr && col < ncols) {
+                const double na = a[e] + acc.v[i][e >> 1][e & 1];
+                ab_a[col * nr + rr] = na;
+                rhs_a[col * nr + rr] = edge ? 0.0 : b[e] + new_ab * na;
+            }
+        }
+    }
 }
 
 // The same in the finite-difference mode, where the grid operator is D_1 (Finalize_EMF's FD
@@ -819,16 +829,14 @@ __global__ void __launch_bounds__(256) emf_band_kernel(const double* __restrict_
     rhs_a[i] = (rr == 0 || rr == nr - 1) ? 0.0 : rhs_a[i] + new_ab * na;
 }
 
-void launch_rlm_b_mag(Ctx& c, double new_ab) {
-    const long total = c.d.nlm * c.d.nr;
-    rlm_b_mag_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c.stream>>>(
-        c.d_s2b, c.d_ab, c.d_rhs_c, c.d_xemf, c.d.nlm, c.d.nr, c.d.L, new_ab, c.nfb, c.d_status);
-    RA_CUDA(cudaGetLastError());
+void launch_emf_radial(Ctx& c, double new_ab) {
     const long ncols = 2 * c.d.nlm;
     double* ab_a = c.d_ab + 5 * c.d.nlm * 2 * c.d.nr;
     if (c.cfg.chebyshev) {
-        dim3 grid((unsigned)((ncols + Sq::BN - 1) / Sq::BN), (unsigned)((c.d.nr + Sq::BM - 1) / Sq::BM));
-        emf_radial_kernel<<<grid, GEMM_THREADS, 0, c.stream>>>(c.d_Memf, c.d_xemf, ab_a, c.d_rhs_a, c.d.nr, ncols,
+        dim3 grid((unsigned)((ncols + GA_BN - 1) / GA_BN), (unsigned)((c.d.nr + GA_BM - 1) / GA_BM));
+        const size_t sm = ga_smem<OperandK, OperandK>();
+        RA_CUDA(cudaFuncSetAttribute(emf_radial_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        emf_radial_kernel<<<grid, GEMM_THREADS, sm, c.stream>>>(c.d_Memf, c.d_xemf, ab_a, c.d_rhs_a, c.d.nr, ncols,
                                                              new_ab);
     } else {
         const long total = ncols * c.d.nr;
@@ -836,7 +844,7 @@ void launch_rlm_b_mag(Ctx& c, double new_ab) {
                                                                              c.d_rhs_a, c.d.nr, ncols, new_ab);
     }
     RA_CUDA(cudaGetLastError());
-    c.launches += 2;
+    ++c.launches;
 }
 
 }  // namespace ra

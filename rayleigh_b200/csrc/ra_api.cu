@@ -974,7 +974,6 @@ static void run_stage(Ctx& c, int k, double new_ab, double old_ab) {
         case 0: launch_cheb_synthesis(c); break;
         case 1:
             launch_post_assemble(c, old_ab);
-            if (c.mag) launch_post_assemble_mag(c, old_ab);
             break;
         case 2:
             launch_rlm_a(c);   // with the magnetic fields when c.mag
@@ -997,7 +996,7 @@ static void run_stage(Ctx& c, int k, double new_ab, double old_ab) {
             break;
         case 6:
             launch_rlm_b(c, new_ab);
-            if (c.mag) launch_rlm_b_mag(c, new_ab);
+            if (c.mag) launch_emf_radial(c, new_ab);
             break;
         default:
             if (c.mixed_solve) {

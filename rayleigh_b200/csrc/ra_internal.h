@@ -318,8 +318,7 @@ void launch_rows_pair(Ctx& c, bool to_rows, double* p2, double* rows, int nfr);
 void lt_forward_prepare(Ctx& c);
 void solve_prepare(Ctx& c);
 void launch_rlm_b(Ctx& c, double new_ab);
-void launch_post_assemble_mag(Ctx& c, double old_ab);
-void launch_rlm_b_mag(Ctx& c, double new_ab);
+void launch_emf_radial(Ctx& c, double new_ab);
 void launch_solve(Ctx& c, bool magnetic);
 void factor_matrices(Ctx& c);
 void rebuild_solve_tiles(Ctx& c);   // LU of the loaded per-l matrices (+ explicit inverses in the mixed form)
