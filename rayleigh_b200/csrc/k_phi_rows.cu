@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(G* M / 4) rows_c2r_kernel(PhysParams P, double
 #pragma unroll
     for (int b = 0; b < ROW_NB; ++b) fo[b] = min(b, max(nfr - 1 - fr0, 0));   // past the last column: any, not stored
     double2 y[4][4];
-    pair_c2r<M, ROW_NB>(P, base, fr0 < nfr ? P.L : 0, fo, dp, buf, tt, y);
+    pair_c2r<M, ROW_NB, false>(P, base, fr0 < nfr ? P.L : 0, fo, dp, buf, tt, y);
     __syncthreads();   // every point is in registers
     const int n0 = R::natural(tt);
 #pragma unroll

@@ -78,6 +78,12 @@ __device__ __forceinline__ void pair_r2c(const PhysParams& P, double* __restrict
 template <int M, int G, int MINB, bool MAG, bool HEAT>
 __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams P) {
     constexpr int T = Pair<M>::T, NT = G * T, NTH = M / 2;
+    // The next batch's spectra come in under this one's terms, except in the largest plans (two radix-8
+    // mid passes): with both the staging and up to six transforms inlined their code outgrows the
+    // instruction cache (M = 1536 with B, N_r = 96: 16.2 ms staged, 12.3 direct; M = 768 with B and
+    // heating, N_r = 128: 3.81 / 3.83 ms, M = 384 with heating 588 / 667 us, with B, N_r = 64,
+    // 451 / 515, M = 256 195 / 218).
+    constexpr bool STAGED = Pair<M>::R1 < 8;
     static_assert(NT % 32 == 0, "whole warps");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ double red[NT / 32];
@@ -130,7 +136,12 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[3] = {A_VR, A_VT, A_VP};
             const bool dp[3] = {false, false, false};
-            pair_c2r<M, 3>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) pair_stage<M, 3>(P, rowbase, L, fo, buf, tt);
+            pair_c2r<M, 3, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) {
+                const int next[4] = {A_DVRDT, A_VR, A_DVTDR, A_DVPDR};
+                pair_stage<M, 4>(P, rowbase, L, next, buf, tt);
+            }
             const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], dlnrho = rowc[RC_DLNRHO];
             const double cs = rowc[RC_CS], sn = rowc[RC_SN], csc = rowc[RC_CSC], cot = rowc[RC_COT], cor = rowc[RC_COR];
             auto w0 = [&](double b, double c) { return rho * (rad * b * b + rad * c * c + cor * sn * rad * rad * c); };
@@ -151,7 +162,11 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[4] = {A_DVRDT, A_VR, A_DVTDR, A_DVPDR};
             const bool dp[4] = {false, true, false, false};
-            pair_c2r<M, 4>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 4, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) {
+                const int next[4] = {A_VP, A_OMR, A_VT, A_DVRDR};
+                pair_stage<M, 4>(P, rowbase, L, next, buf, tt);
+            }
             const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], csc = rowc[RC_CSC];
             const double dlnrho = rowc[RC_DLNRHO], vh = rowc[RC_VH];
             // a = sin(theta) dv_r/dtheta, b = dv_r/dphi, c = sin(theta) dv_theta/dr, d = sin(theta) dv_phi/dr
@@ -181,7 +196,11 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[4] = {A_VP, A_OMR, A_VT, A_DVRDR};
             const bool dp[4] = {true, false, true, false};
-            pair_c2r<M, 4>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 4, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) {
+                const int next[3] = {A_DTDR, A_DTDT, A_T};
+                pair_stage<M, 3>(P, rowbase, L, next, buf, tt);
+            }
             const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], csc = rowc[RC_CSC];
             const double cot = rowc[RC_COT], c2r = rowc[RC_C2R], dlnrho = rowc[RC_DLNRHO], vh = rowc[RC_VH];
             const double csc2 = csc * csc;
@@ -212,7 +231,11 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[3] = {A_DTDR, A_DTDT, A_T};
             const bool dp[3] = {false, false, true};
-            pair_c2r<M, 3>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 3, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED && MAG) {
+                const int next[4] = {A_BR, A_BT, A_BP, A_CBR};
+                pair_stage<M, 4>(P, rowbase, L, next, buf, tt);
+            }
             const double csc = rowc[RC_CSC], orad = rowc[RC_ORAD];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -227,7 +250,12 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[4] = {A_VR, A_VT, A_VP, A_DVRDR};
             const bool dp[4] = {false, false, false, false};
-            pair_c2r<M, 4>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) pair_stage<M, 4>(P, rowbase, L, fo, buf, tt);
+            pair_c2r<M, 4, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) {
+                const int next[4] = {A_DVRDT, A_VR, A_DVTDR, A_VT};
+                pair_stage<M, 4>(P, rowbase, L, next, buf, tt);
+            }
             const double rad = rowc[RC_RAD], orad = rowc[RC_ORAD], rho = rowc[RC_RHO], dlnrho = rowc[RC_DLNRHO];
             const double cs = rowc[RC_CS], sn = rowc[RC_SN], csc = rowc[RC_CSC], cot = rowc[RC_COT], cor = rowc[RC_COR];
             auto w0 = [&](double a, double b, double c, double xx) {
@@ -253,7 +281,11 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[4] = {A_DVRDT, A_VR, A_DVTDR, A_VT};
             const bool dp[4] = {false, true, false, true};
-            pair_c2r<M, 4>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 4, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) {
+                const int next[4] = {A_DVPDR, A_VP, A_OMR, A_DTDR};
+                pair_stage<M, 4>(P, rowbase, L, next, buf, tt);
+            }
             const double rad = rowc[RC_RAD], rho = rowc[RC_RHO], csc = rowc[RC_CSC], c2r = rowc[RC_C2R];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -273,7 +305,11 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[4] = {A_DVPDR, A_VP, A_OMR, A_DTDR};
             const bool dp[4] = {false, true, false, false};
-            pair_c2r<M, 4>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 4, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) {
+                const int next[2] = {A_DTDT, A_T};
+                pair_stage<M, 2>(P, rowbase, L, next, buf, tt);
+            }
             const double csc = rowc[RC_CSC], c2r = rowc[RC_C2R];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -291,7 +327,11 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[2] = {A_DTDT, A_T};
             const bool dp[2] = {false, true};
-            pair_c2r<M, 2>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 2, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED && MAG) {
+                const int next[4] = {A_BR, A_BT, A_BP, A_CBR};
+                pair_stage<M, 4>(P, rowbase, L, next, buf, tt);
+            }
             const double csc = rowc[RC_CSC], orad = rowc[RC_ORAD];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -325,7 +365,7 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[4] = {A_BR, A_BT, A_BP, A_CBR};
             const bool dp[4] = {false, false, false, false};
-            pair_c2r<M, 4>(P, rowbase, L, fo, dp, buf, tt, y);
+            pair_c2r<M, 4, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
             const double csc = rowc[RC_CSC], rad = rowc[RC_RAD], rho = rowc[RC_RHO];
             // the Alfven speed (:798-806)
             const double hfb = P.llmax * orad * orad / rho * P.lorentz, rfb = P.lorentz / (dr * dr * rho);
@@ -366,7 +406,8 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
         {
             const int fo[2] = {A_CBT, A_CBP};
             const bool dp[2] = {false, false};
-            pair_c2r<M, 2>(P, rowbase, L, fo, dp, buf, tt, y);
+            if constexpr (STAGED) pair_stage<M, 2>(P, rowbase, L, fo, buf, tt);
+            pair_c2r<M, 2, STAGED>(P, rowbase, L, fo, dp, buf, tt, y);
             const double csc = rowc[RC_CSC], rad = rowc[RC_RAD], rho = rowc[RC_RHO];
             const double lc = P.lorentz, r2lc = rad * rad * lc, lcr = lc / rho;
 #pragma unroll

@@ -178,13 +178,10 @@ __device__ __forceinline__ void mid_barrier(int tt) {
     }
 }
 
-// c2r of NB fields of this row pair (fields fo[b], d/dphi where dp[b]); on return y[b][i] holds the
-// (south, north) values of field b at the row's point 4 tt + i (digit-reversed order).  L is 0 for
-// a row past the last radius.
+// The first pass of NB fields (fo[b], d/dphi where dp[b]) straight from global memory.
 template <int M, int NB>
-__device__ __forceinline__ void pair_c2r(const PhysParams& P, const double* __restrict__ rowbase, int L,
-                                         const int (&fo)[NB], const bool (&dp)[NB], double2* buf, int tt,
-                                         double2 (&y)[4][4]) {
+__device__ __forceinline__ void pair_first(const PhysParams& P, const double* __restrict__ rowbase, int L,
+                                           const int (&fo)[NB], const bool (&dp)[NB], double2* buf, int tt) {
     using S = Pair<M>;
     constexpr int F = S::F, Q = S::Q, T = S::T, NITEM = NB * (Q / 2);
     const long ostride = (long)P.ncola, mstride = 2L * P.ncola;
@@ -247,6 +244,113 @@ __device__ __forceinline__ void pair_c2r(const PhysParams& P, const double* __re
             if (j + 1 < F) wj = cmul(wj, w);
         }
     }
+}
+
+// The spectra of NB fields (fo[b]) on their way into the FFT buffer by cp.async: E_m of field b in slot
+// b M + m, O_m in slot b M + M/2 + m, m < L (0 for a row past the last radius).  The caller's use of
+// the buffer ends with the barrier in here.  Called as soon as the previous batch has left the buffer,
+// it brings the next one in under the nonlinear terms; loads into registers were held up by the small
+// L1 that 197 KB of shared memory leave (their sectors in flight have to fit it).
+template <int M, int NB>
+__device__ __forceinline__ void pair_stage(const PhysParams& P, const double* __restrict__ rowbase, int L,
+                                           const int (&fo)[NB], double2* buf, int tt) {
+    const long ostride = (long)P.ncola, mstride = 2L * P.ncola;
+    const unsigned s0 = (unsigned)__cvta_generic_to_shared(buf);
+    __syncthreads();
+    // eight consecutive m of one field, then the batch's other fields (their records share cache lines),
+    // then the other parity
+    const int n = 2 * NB * ((L + 7) & ~7);
+    for (int e = tt; e < n; e += Pair<M>::T) {
+        const int b = (e >> 3) % NB, hi = e / (8 * NB), par = hi & 1, m = (hi >> 1) * 8 + (e & 7);
+        int f = fo[0];
+#pragma unroll
+        for (int i = 1; i < NB; ++i)
+            if (b == i) f = fo[i];
+        if (m < L)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s0 + 16 * (b * M + par * (M / 2) + m)),
+                         "l"(rowbase + m * mstride + par * ostride + 2 * f)
+                         : "memory");
+    }
+}
+
+// The first pass of NB fields whose spectra pair_stage brought (d/dphi where dp[b]).
+template <int M, int NB>
+__device__ __forceinline__ void pair_first_staged(const PhysParams& P, int L, const bool (&dp)[NB], double2* buf,
+                                                  int tt) {
+    using S = Pair<M>;
+    constexpr int F = S::F, Q = S::Q, T = S::T, H = Q / 2;
+    static_assert(2 * H <= T, "one item of a field pair per thread");
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    unsigned dphi = 0;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) dphi |= dp[b] ? 1u << b : 0u;
+    // two fields at a time: every thread takes its item's values, and after the barrier the fields'
+    // transforms replace them (one copy of the code for both pairs: the kernel, with up to six
+    // transforms inlined, has to stay inside the instruction cache)
+#pragma unroll 1
+    for (int b0 = 0; b0 < NB; b0 += 2) {
+        const int nf = NB - b0 < 2 ? 1 : 2;
+        const bool active = tt < nf * H;
+        const int b = b0 + (tt >= H ? 1 : 0), k = tt - (tt >= H ? H : 0);
+        const bool self = k == 0;
+        const int kp = self ? Q / 2 : Q - k;
+        double2* fb = buf + b * M;
+        const int idx[4] = {k, k + Q, kp, kp + Q};
+        const double2 zero = make_double2(0.0, 0.0);
+        double2 zp[4], zm[4], xp = zero, xm = zero, w = zero;
+        if (active) {
+            const bool d = (dphi >> b) & 1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                double2 e = zero, o = zero;
+                if (idx[i] < L) {
+                    e = fb[idx[i]];
+                    o = fb[M / 2 + idx[i]];
+                }
+                hemispheres(e, o, idx[i], d, zp[i], zm[i]);
+            }
+            if (F == 6 && self && 2 * Q < L) hemispheres(fb[2 * Q], fb[M / 2 + 2 * Q], 2 * Q, d, xp, xm);
+            w = __ldg(P.wr + (self ? kp : k));   // exp(2 pi i k / M)
+        }
+        __syncthreads();
+        if (active) {
+            double2 ya[F], yb[F];
+            dft_from4<F, 1>(zp[0], zp[1], self ? xm : zm[3], self ? zm[1] : zm[2], ya);
+            if (F == 6 && self) {   // m = M/3 = l_max: inputs 2 (here) and 4 (above) of residue 0
+                const double S3 = 0.86602540378443864676;
+                const double2 x1 = make_double2(-0.5 * xp.x - S3 * xp.y, -0.5 * xp.y + S3 * xp.x);
+                const double2 x2 = make_double2(-0.5 * xp.x + S3 * xp.y, -0.5 * xp.y - S3 * xp.x);
+#pragma unroll
+                for (int j = 0; j < F; ++j) ya[j] = cadd(ya[j], j % 3 == 0 ? xp : (j % 3 == 1 ? x1 : x2));
+            }
+            dft_from4<F, -1>(self ? zm[2] : zm[0], self ? zm[3] : zm[1], zp[3], zp[2], yb);
+            fb[swz<M>(k)] = ya[0];
+            fb[swz<M>(kp)] = yb[0];
+            double2 wj = w;
+#pragma unroll
+            for (int j = 1; j < F; ++j) {
+                fb[swz<M>(j * Q + k)] = self ? ya[j] : cmul(ya[j], wj);
+                fb[swz<M>(j * Q + kp)] = cmul(yb[j], cconj(wj));
+                if (j + 1 < F) wj = cmul(wj, w);
+            }
+        }
+    }
+}
+
+// c2r of NB fields of this row pair (fields fo[b], d/dphi where dp[b]; STAGED: the spectra are on their
+// way by pair_stage); on return y[b][i] holds the (south, north) values of field b at the row's point
+// 4 tt + i (digit-reversed order).  L is 0 for a row past the last radius.
+template <int M, int NB, bool STAGED>
+__device__ __forceinline__ void pair_c2r(const PhysParams& P, const double* __restrict__ rowbase, int L,
+                                         const int (&fo)[NB], const bool (&dp)[NB], double2* buf, int tt,
+                                         double2 (&y)[4][4]) {
+    using S = Pair<M>;
+    constexpr int Q = S::Q;
+    if constexpr (STAGED)
+        pair_first_staged<M, NB>(P, L, dp, buf, tt);
+    else
+        pair_first<M, NB>(P, rowbase, L, fo, dp, buf, tt);
     __syncthreads();
     if constexpr (S::R1 > 1) {
         pair_mid_pass<M, NB, S::R1, Q, false>(buf, P.twq, tt);
