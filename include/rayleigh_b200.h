@@ -565,7 +565,7 @@ int ra_fft_c2r(ra_ctx* ctx, double* x, long howmany);
  *   d_grid: [n_theta][nfr][n_phi + 2] real rows (Gauss-Legendre theta order)
  *   d_work: l_max + 1 times n_theta times nfr complex entries (the E/O or folded blocks)
  * stage_ms (may be NULL) receives the device times of [0] the Legendre product (with the
- * digit split), [1] the relayout and [2] the FFT.  The call first makes the context's stream
+ * digit split), [1] the relayout (0 where one kernel does both) and [2] the FFT.  The call first makes the context's stream
  * wait for the work queued on the legacy default stream (operands written there are
  * complete) and returns with its own work complete; operands written on other streams must
  * be complete before the call. */

@@ -6,7 +6,8 @@
 // l of one parity, 128 on average at l_max = 511, so that a tile is only eight k-tiles long: the
 // copies of the next two k-tiles are in flight without holding registers, one barrier serves a
 // k-tile, and fragments are read in 16-byte pieces, half the shared-memory instructions of
-// element-wise ones: a lane's two neighbouring rows (or columns) belong to two mma tiles, so that the
+// element-wise ones (l_max 511, N_r 96 with B: inverse 12.63 -> 10.73 ms, 0.86 of DGEMM, forward 5.67 ->
+// 5.12): a lane's two neighbouring rows (or columns) belong to two mma tiles, so that the
 // tile's rows and columns come out permuted (acc_each knows the order), four neighbouring columns a lane.
 #pragma once
 

@@ -7,7 +7,8 @@
 //
 // What bounds them: HBM.  Each direction reads its input once and writes its output once, where
 // the separate relayout and in-place FFT moved the rows three times and the FFT, one row per CTA
-// with a twiddle table copied to shared memory for each, ran at a fifth of the HBM rate.
+// with a twiddle table copied to shared memory for each, ran at a fifth of the HBM rate (l_max 255, 512
+// columns, FP64 inverse call: 3303 -> 1130 us).
 // The rows enter and leave in natural phi order: the points of the last pass, digit-reversed, go
 // through shared memory once more, at natural index n plus one slot per F R1 points, which
 // spreads the 8 lanes of a phase (their n differ by F R1) over the 8 banks.
