@@ -36,19 +36,6 @@ __device__ __forceinline__ double2 twiddle(const double2* wr, int N, int e, int 
     return w;
 }
 
-// The same from a table in global memory (read-only path).
-__device__ __forceinline__ double2 twiddle_g(const double2* __restrict__ wr, int N, int e, int sign) {
-    double2 w;
-    if (2 * e < N) {
-        w = __ldg(wr + 2 * e);
-    } else {
-        const double2 v = __ldg(wr + 2 * e - N);
-        w = make_double2(-v.x, -v.y);
-    }
-    if (sign < 0) w.y = -w.y;
-    return w;
-}
-
 // Runs nb independent FFTs of length N stored at a + b*N (b < nb), scratch at
 // bb + b*N; returns the buffer base holding the results.  Must be entered with
 // a synchronised input; leaves the result synchronised.
@@ -389,34 +376,6 @@ __device__ __forceinline__ void row_c2r(const PhysParams& P, const double* __res
             const int n = t + q * row_threads(N);
             y[b][q] = (n < N) ? buf[SW(b * FS + n)] : make_double2(0.0, 0.0);
         }
-}
-
-// X_k of the real transform from the complex r2c output Z (in place, one (k, N-k) pair per
-// work item): X_k = e - i conj(w^k) d with e, d the half sums / differences of Z_k and
-// conj Z_{N-k}, each times hs(f); Im X_0 = 0; only k < L is kept.
-template <int N, class HS>
-__device__ __forceinline__ void r2c_finish(double2* a, int nf, int L, const double2* __restrict__ wr, int t,
-                                           const HS& hsf) {
-    constexpr int FS = fstride(N);
-    constexpr int NI = N / 2 + 1;
-    for (int g = t; g < nf * NI; g += row_threads(N)) {
-        const int f = g / NI, k = g - f * NI;
-        const double2 zk = a[SW(f * FS + k)];
-        const double2 zn = a[SW(f * FS + (N - k) % N)];
-        const double2 wk = __ldg(wr + k);   // w^(N-k) = -conj(w^k)
-        const double hs = hsf(f);
-        auto xval = [&](double2 p, double2 q, double2 w, bool zero_im) {   // X from Z_kk = p, Z_{N-kk} = q
-            const double2 qn = cconj(q);
-            const double2 e = make_double2(hs * (p.x + qn.x), hs * (p.y + qn.y));
-            const double2 d = make_double2(hs * (p.x - qn.x), hs * (p.y - qn.y));
-            const double2 wd = cmul(cconj(w), d);
-            double2 X = make_double2(e.x + wd.y, e.y - wd.x);
-            if (zero_im) X.y = 0.0;
-            return X;
-        };
-        if (k < L) a[SW(f * FS + k)] = xval(zk, zn, wk, k == 0);
-        if (k != 0 && 2 * k != N && N - k < L) a[SW(f * FS + N - k)] = xval(zn, zk, make_double2(-wk.x, wk.y), false);
-    }
 }
 
 FFTPlan make_plan(int n) {
