@@ -345,10 +345,16 @@ __global__ void __launch_bounds__(256) lu_offdiag_kernel(double* __restrict__ ma
 // columns arrive by 8-byte cp.async, all in flight together (one load a column
 // after the other took longer than the substitution below n ~ 200), and every
 // system of the step goes out as one launch where two CTAs fit an SM (n <= 384).
-// Without a shared-memory ring for M the block takes 65 KB at n = 144 (three CTAs
-// per SM instead of one) and 114 KB at n = 384 (two): 71 -> 27 us a step at n = 144, l_max 41, 566 -> 304
+// Without a shared-memory ring for M the block takes 65 KB at n = 144 and 114 KB at n = 384: two CTAs
+// an SM (126 registers allow no more) instead of one: 71 -> 27 us a step at n = 144, l_max 41, 566 -> 304
 // at n = 384, l_max 127, 8.02 -> 4.11 ms at n = 288, l_max 511 with B.
+// Above n = 384 a CTA has its SM to itself, or shares it on large grids only (16 columns, n <= 832), and
+// waits for rows of M that come from HBM: 16 systems of n = 576, which stay in L2, take 150 us and 64 take
+// 204; two or four more chunks in registers change nothing.  There (LONG) each warp prefetches its chunks
+// into L2 eight ahead: n = 576 204 -> 170 us, 1152 618 -> 454 (64 systems, one column), W-P-T and Z at
+// N_r = 192, l_max 127 908 -> 754 us.  Below, two CTAs hide it: N_r = 64, l_max 255 with B 519 us without, 532 with.
 constexpr int LS_KC = 16;                 // K per chunk
+constexpr int LS_AHEAD = 8;               // chunks a warp's prefetches run ahead
 constexpr int LS_WARPS = 8, LS_THREADS = 32 * LS_WARPS;
 
 __device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
@@ -380,7 +386,7 @@ struct LuSolveShape {
     }
 };
 
-template <int NC>
+template <int NC, bool LONG>
 __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4* __restrict__ tiles, LuSysSet set,
                                                                       int mode, int ncols_fixed) {
     constexpr int NT = NC / 8;               // n-tiles per warp
@@ -442,6 +448,27 @@ __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4
             }
         }
     };
+    int p_bw = 0, p_q = 0, p_j = grp;                      // the same for the prefetches
+    auto prefetch = [&] {                                  // both ends of the chunk's 16 row pieces
+        if (LONG && p_bw < 2) {
+            const bool bw = p_bw == 1;
+            const int ib = bw ? nblk - 1 - p_q : p_q;
+            const int gr = ib * SB + rgp * 16 + (lane & 15);
+            const int gk = (bw ? ib * SB : 0) + p_j * LS_KC + (lane >> 4) * (LS_KC - 1);
+            if (gr < n && gk < n) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(M + (size_t)gr * n + gk));
+            p_j += 2;
+            if (p_j >= nchunks(bw, ib)) {
+                p_j = grp;
+                if (++p_q == nblk) {
+                    p_q = 0;
+                    ++p_bw;
+                }
+            }
+        }
+    };
+    if (LONG)
+#pragma unroll 1
+        for (int i = 0; i < LS_AHEAD; ++i) prefetch();
     double a0[2][4] = {}, a1[2][4] = {};
     fetch(a0);
     fetch(a1);
@@ -507,8 +534,10 @@ __global__ void __launch_bounds__(LS_THREADS, 2) lu_substitute_kernel(const int4
                 }
             };
             for (int j = grp; j < nch; j += 4) {   // an even number of chunks per group
+                prefetch();
                 multiply(a0, j);
                 fetch(a0);
+                prefetch();
                 multiply(a1, j + 2);
                 fetch(a1);
             }
@@ -729,10 +758,11 @@ void launch_lu_solve(cudaStream_t st, const int* d_tiles, int ntiles, const LuSy
         set_smem(kern, sm);
         kern<<<ntiles, LS_THREADS, sm, st>>>(reinterpret_cast<const int4*>(d_tiles), set, mode, ncols_fixed);
     };
+    const bool big = n > 384;   // LONG: see the kernel's comment
     if (nc == 32)
-        go(lu_substitute_kernel<32>, LuSolveShape<32>::smem(n));
+        go(big ? lu_substitute_kernel<32, true> : lu_substitute_kernel<32, false>, LuSolveShape<32>::smem(n));
     else
-        go(lu_substitute_kernel<16>, LuSolveShape<16>::smem(n));
+        go(big ? lu_substitute_kernel<16, true> : lu_substitute_kernel<16, false>, LuSolveShape<16>::smem(n));
     RA_CUDA(cudaGetLastError());
 }
 
@@ -852,8 +882,8 @@ void factor_matrices(Ctx& c) {
 
 // Implicit_Solve (Linear_Solve.F90:423-457): x = A_l^-1 b for every (system, l): W-P-T and Z, and
 // with magnetic the C and A equations (l = 0 is the identity there).  One launch where its shared
-// memory (set by the W-P-T columns) still lets two CTAs share an SM, n <= 384; above that the small
-// systems go out on their own, three CTAs an SM.
+// memory (set by the W-P-T columns) still lets two CTAs share an SM, n <= 384; above that the W-P-T block
+// takes an SM for itself, and the small systems go out on their own, two CTAs an SM.
 void launch_solve(Ctx& c, bool magnetic) {
     if (!c.d_solve_tiles) throw ArgError("solve tiles not prepared (solve_prepare runs at set-up)");
     const int nr = c.d.nr, rest = c.n_solve_tiles_z * (magnetic ? 3 : 1);
