@@ -829,7 +829,7 @@ __global__ void fft_rows_kernel(double* x, long howmany, const double2* wrg, FFT
 void launch_fft_rows(Ctx& c, double* d_x, long howmany, int inverse) {
     FFTPlan plan = make_plan(c.d.nth);
     const size_t smem = 3 * (size_t)c.d.nth * sizeof(double2);
-    RA_CUDA(cudaFuncSetAttribute(fft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(fft_rows_kernel);
     fft_rows_kernel<<<(unsigned)howmany, 256, smem, c.stream>>>(d_x, howmany, reinterpret_cast<const double2*>(c.d_twid),
                                                               plan, inverse);
     RA_CUDA(cudaGetLastError());

@@ -720,12 +720,12 @@ int lu_factor_batch(cudaStream_t st, LuWork& w, double* d_mats, int* d_perm, int
     if (n < 2 || (n & 1)) throw ArgError("per-l matrices must have an even order >= 2");
     lu_workspace(w, n, count);
     const int nblk = (n + SB - 1) / SB;
-    if (LuFactorSmem<32>::bytes(n) <= (size_t)(227 << 10)) {
-        set_smem(lu_factor_kernel<32>, LuFactorSmem<32>::bytes(n));
+    if (LuFactorSmem<32>::bytes(n) <= (size_t)SMEM_BLOCK) {
+        allow_shared(lu_factor_kernel<32>);
         lu_factor_kernel<32><<<count, LU_THREADS, LuFactorSmem<32>::bytes(n), st>>>(d_mats, n, d_skip, d_perm,
                                                                                    w.d_status);
-    } else if (LuFactorSmem<16>::bytes(n) <= (size_t)(227 << 10)) {
-        set_smem(lu_factor_kernel<16>, LuFactorSmem<16>::bytes(n));
+    } else if (LuFactorSmem<16>::bytes(n) <= (size_t)SMEM_BLOCK) {
+        allow_shared(lu_factor_kernel<16>);
         lu_factor_kernel<16><<<count, LU_THREADS, LuFactorSmem<16>::bytes(n), st>>>(d_mats, n, d_skip, d_perm,
                                                                                    w.d_status);
     } else {
@@ -755,7 +755,7 @@ void launch_lu_solve(cudaStream_t st, const int* d_tiles, int ntiles, const LuSy
     for (int i = 0; i < set.count; ++i) n = std::max(n, set.s[i].n);
     if (n > LS_MAX_N) throw ArgError("per-l matrix order too large for the block substitution");
     auto go = [&](auto kern, size_t sm) {
-        set_smem(kern, sm);
+        allow_shared(kern);
         kern<<<ntiles, LS_THREADS, sm, st>>>(reinterpret_cast<const int4*>(d_tiles), set, mode, ncols_fixed);
     };
     const bool big = n > 384;   // LONG: see the kernel's comment
@@ -782,8 +782,8 @@ void launch_lu_refine(cudaStream_t st, const int* d_tiles, int ntiles, const LuS
     const int nrow = (s.n + SB - 1) / SB * SB;
     const size_t sm = (size_t)nrow * RF_NC * sizeof(double) + (size_t)nrow * RF_NC * sizeof(float) +
                       (size_t)SB * RF_NC * sizeof(float);
-    if (sm > (size_t)(227 << 10)) throw ArgError("per-l matrix order too large for the refinement kernel");
-    set_smem(lu_refine_kernel, sm);
+    if (sm > (size_t)SMEM_BLOCK) throw ArgError("per-l matrix order too large for the refinement kernel");
+    allow_shared(lu_refine_kernel);
     lu_refine_kernel<<<ntiles, RF_THREADS, sm, st>>>(reinterpret_cast<const int4*>(d_tiles), s, d_mf, d_a, ncols,
                                                      d_iters);
     RA_CUDA(cudaGetLastError());

@@ -241,7 +241,7 @@ void launch_cheb_synthesis(Ctx& c) {
     const long ncols = 2 * c.d.nlm;
     const size_t smem = ((size_t)CH_COLS * cheb_ldb(c.d.kc) + CH_STAGES * CH_ROWS * CH_LDA) * sizeof(double);
     // the limit is per device: set it on every launch (a host-side call, also legal during capture)
-    RA_CUDA(cudaFuncSetAttribute(cheb_synthesis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared(cheb_synthesis_kernel);
     // Where the (tile, field) CTAs leave SMs without three of them, the derivative orders go to CTAs of
     // their own: the chain of up to four orders is what a small grid waits for.
     dim3 grid((unsigned)((ncols + CH_COLS - 1) / CH_COLS), c.mag ? 6 : 4);

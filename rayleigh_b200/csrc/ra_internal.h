@@ -348,6 +348,8 @@ void launch_lt_forward_mixed(Ctx& c);
 void launch_solve_mixed(Ctx& c);
 void mixed_resplit_solve(Ctx& c);
 
+constexpr int SMEM_BLOCK = 227 << 10;   // shared memory a block may have, static and dynamic
+
 #define RA_CUDA(call)                                                             \
     do {                                                                          \
         cudaError_t e_ = (call);                                                  \
@@ -363,6 +365,16 @@ struct CudaError {
         what = std::string(call) + " failed at " + file + ":" + std::to_string(line) + ": " + cudaGetErrorString(e);
     }
 };
+
+// Lets a kernel whose shared memory grows with the problem take all that a block may have.  The limit
+// belongs to the function and is shared by every context on the device: were it one launch's own size,
+// another host thread could lower it between this thread's setting and its launch, which is then refused.
+template <class F>
+inline void allow_shared(F* kern) {
+    cudaFuncAttributes a;
+    RA_CUDA(cudaFuncGetAttributes(&a, kern));
+    RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BLOCK - (int)a.sharedSizeBytes));
+}
 
 struct SingularError {   // a zero pivot in a per-l matrix: RA_ERR_SINGULAR
     std::string what;
