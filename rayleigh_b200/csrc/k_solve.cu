@@ -881,12 +881,12 @@ void factor_matrices(Ctx& c) {
 }
 
 // Implicit_Solve (Linear_Solve.F90:423-457): x = A_l^-1 b for every (system, l): W-P-T and Z, and
-// with magnetic the C and A equations (l = 0 is the identity there).  One launch where its shared
+// with magnetism the C and A equations (l = 0 is the identity there).  One launch where its shared
 // memory (set by the W-P-T columns) still lets two CTAs share an SM, n <= 384; above that the W-P-T block
 // takes an SM for itself, and the small systems go out on their own, two CTAs an SM.
-void launch_solve(Ctx& c, bool magnetic) {
+void launch_solve(Ctx& c) {
     if (!c.d_solve_tiles) throw ArgError("solve tiles not prepared (solve_prepare runs at set-up)");
-    const int nr = c.d.nr, rest = c.n_solve_tiles_z * (magnetic ? 3 : 1);
+    const int nr = c.d.nr, rest = c.n_solve_tiles_z * (c.mag ? 3 : 1);
     const LuSysSet set{{{c.d_Awpt, c.d_perm_wpt, c.d_rhs_wpt, c.d_sol_wpt, 3 * nr},
                         {c.d_Az, c.d_perm_z, c.d_rhs_z, c.d_sol_z, nr},
                         {c.d_Ac, c.d_perm_c, c.d_rhs_c, c.d_sol_c, nr},

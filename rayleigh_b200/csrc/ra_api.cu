@@ -1002,7 +1002,7 @@ static void run_stage(Ctx& c, int k, double new_ab, double old_ab) {
             if (c.mixed_solve) {
                 launch_solve_mixed(c);   // every system, C and A included
             } else {
-                launch_solve(c, c.mag);
+                launch_solve(c);
             }
             break;
     }
@@ -1336,10 +1336,27 @@ static void autotune(Ctx& c, int nreps, double* ms_out) {
         RA_CUDA(cudaMemsetAsync(c.d_p2a, 0, (size_t)c.d.L * c.d.nth * c.nfa * 2 * c.d.nr * sizeof(double), c.stream));
         RA_CUDA(cudaMemsetAsync(c.d_rhs_wpt, 0, 3 * plane * sizeof(double), c.stream));
         RA_CUDA(cudaMemsetAsync(c.d_rhs_z, 0, plane * sizeof(double), c.stream));
+        if (c.mag) {
+            RA_CUDA(cudaMemsetAsync(c.d_rhs_c, 0, plane * sizeof(double), c.stream));
+            RA_CUDA(cudaMemsetAsync(c.d_rhs_a, 0, plane * sizeof(double), c.stream));
+        }
     }
     // the solve overwrites the state: park it in the grid buffer (rebuilt by every step)
-    RA_CUDA(cudaMemcpyAsync(c.d_g, c.d_sol_wpt, 3 * plane * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-    RA_CUDA(cudaMemcpyAsync(c.d_g + 3 * plane, c.d_sol_z, plane * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+    struct Part { double* at; size_t planes; };
+    std::vector<Part> state = {{c.d_sol_wpt, 3}, {c.d_sol_z, 1}};
+    if (c.mag) {
+        state.push_back({c.d_sol_c, 1});
+        state.push_back({c.d_sol_a, 1});
+    }
+    auto move_state = [&](bool back) {
+        double* g = c.d_g;
+        for (const Part& p : state) {
+            RA_CUDA(cudaMemcpyAsync(back ? p.at : g, back ? g : p.at, p.planes * plane * sizeof(double),
+                                    cudaMemcpyDeviceToDevice, c.stream));
+            g += p.planes * plane;
+        }
+    };
+    move_state(false);
     cudaEvent_t e0, e1;
     RA_CUDA(cudaEventCreate(&e0));
     RA_CUDA(cudaEventCreate(&e1));
@@ -1354,7 +1371,7 @@ static void autotune(Ctx& c, int nreps, double* ms_out) {
                     launch_physics(c);
                 } else {
                     if (c.mixed_solve) return;   // the mixed form solves by split products
-                    launch_solve(c, false);
+                    launch_solve(c);
                 }
             };
             run();
@@ -1375,8 +1392,7 @@ static void autotune(Ctx& c, int nreps, double* ms_out) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    RA_CUDA(cudaMemcpyAsync(c.d_sol_wpt, c.d_g, 3 * plane * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
-    RA_CUDA(cudaMemcpyAsync(c.d_sol_z, c.d_g + 3 * plane, plane * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
+    move_state(true);
     RA_CUDA(cudaMemsetAsync(c.d_status, 0, sizeof(int), c.stream));
     RA_CUDA(cudaStreamSynchronize(c.stream));
 }

@@ -319,7 +319,7 @@ void lt_forward_prepare(Ctx& c);
 void solve_prepare(Ctx& c);
 void launch_rlm_b(Ctx& c, double new_ab);
 void launch_emf_radial(Ctx& c, double new_ab);
-void launch_solve(Ctx& c, bool magnetic);
+void launch_solve(Ctx& c);
 void factor_matrices(Ctx& c);
 void rebuild_solve_tiles(Ctx& c);   // LU of the loaded per-l matrices (+ explicit inverses in the mixed form)
 // k_solve.cu
