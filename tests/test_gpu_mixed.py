@@ -161,3 +161,61 @@ def test_mixed_stages_per_lmax(lmax):
     assert max(state.values()) <= MIXED_TOL, errs
     bad = {k: v for k, v in errs.items() if v > 1e-7}
     assert not bad, errs
+
+
+# Legendre products are split ones from l_max 199 on (spectral -> physical) and from 149 on (back): the cases
+# below lie above both lines, or between them, with the fields of the dynamo set, and in the
+# finite-difference mode, whose mixed form has no other split product.
+SPLIT = dict(n_r=10, dt=1e-4, rayleigh=1e5, ekman=1e-3, precision=1)
+SPLIT_MHD = dict(SPLIT, magnetism=True, magnetic_prandtl=5.0)
+
+
+@pytest.mark.parametrize("cfg", [
+    dict(SPLIT_MHD, l_max=255),
+    dict(SPLIT_MHD, l_max=255, chebyshev=False),
+    dict(SPLIT_MHD, l_max=169, n_theta=256),    # forward product split, inverse FP64
+    dict(SPLIT, l_max=170, n_theta=256),
+])
+def test_split_legendre_products_over_steps(cfg):
+    """Five steps against the oracle: 1e-9 (relative L2 per field), the bound of every mixed run.
+    Measured: at most 2.1e-10 (Z)."""
+    import oracle as O
+    import test_gpu_mhd as M
+    oc = M._ocfg(cfg)
+    mag = bool(cfg.get("magnetism"))
+    o = O.Oracle(oc)
+    wpt, z, c, a = M._seed(oc)
+    o.init_state(wpt, z, c_coeffs=c if mag else None, a_coeffs=a if mag else None)
+    g = M._ctx(cfg)
+    g.put_state(wpt, z, None, iteration=1)
+    if mag:
+        g.put_magnetic_state(c, a)
+    for _ in range(5):
+        o.step()
+    g.step(5)
+    if mag:
+        errs = M._state_errs(o, g)
+    else:
+        w, zz, _ = g.get_state()
+        ref = _fields(o.rhs_wpt, o.rhs_z, oc.n_r)
+        errs = {k: _rel(v, ref[k]) for k, v in _fields(w, zz, oc.n_r).items()}
+    print(cfg, {k: f"{v:.2e}" for k, v in errs.items()})
+    assert max(errs.values()) < MIXED_TOL, errs
+    g.close()
+
+
+@pytest.mark.parametrize("grid", [dict(l_max=255), dict(l_max=169, n_theta=256)])
+def test_split_stages_with_magnetism(grid):
+    """The second step's stages with the 17 fields in and 7 out of the dynamo set: every buffer to 1e-7 of
+    its own norm as above, the solution to 1e-9 but for Z, which started from rest one step before.  It is
+    all nonlinear term then: the split products' error, 2^-40 of a column's maximum at every l, reaches it
+    through a curl, which multiplies by l, so that the 1e-11 of the transforms becomes 1.2e-9 of the
+    low-l Z at l_max 255 (1.2e-11 at 63; 1.4e-10 after ten steps): 1e-8 for Z."""
+    import test_gpu_mhd as M
+    errs = M._stage_compare(dict(SPLIT_MHD, n_r=8, dt=1e-6, **grid), steps_before=1)
+    print(grid, {k: f"{v:.2e}" for k, v in errs.items()})
+    state = {k: v for k, v in errs.items() if k.startswith("sol_")}
+    assert max(v for k, v in state.items() if k != "sol_Z") <= MIXED_TOL, errs
+    assert state["sol_Z"] <= 1e-8, errs
+    bad = {k: v for k, v in errs.items() if v > 1e-7}
+    assert not bad, errs
