@@ -36,7 +36,13 @@ def test_magnetic_stages(n_theta, n_r):
                                  ekman=1e-3, magnetism=True, magnetic_prandtl=5.0), steps_before=1))
 
 
-@pytest.mark.parametrize("n_theta,n_r", [(32, 10), (48, 10), (192, 16), (256, 16)])
+@pytest.mark.parametrize("top", [0, 1])
+def test_hydro_stages_512(top):
+    _check(H._stage_compare(dict(n_r=8, l_max=340 + top, n_theta=512, dt=1e-6, rayleigh=1e5, ekman=1e-3),
+                            steps_before=1))
+
+
+@pytest.mark.parametrize("n_theta,n_r", [(32, 10), (48, 10), (192, 16), (256, 16), (512, 8), (768, 8)])
 @pytest.mark.parametrize("mag", [False, True])
 def test_heating_stages(n_theta, n_r, mag):
     compare = M._stage_compare if mag else H._stage_compare
