@@ -547,19 +547,11 @@ void ozaki_split(Ctx& c, const OzSplitJob* d_jobs, int njobs, int max_rows, int 
     }
 }
 
-// SM count of the current device (asked on every call: one process may drive several devices)
-static int oz_sm_count() {
-    int dev = 0, n = 0;
-    RA_CUDA(cudaGetDevice(&dev));
-    RA_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-    return n;
-}
-
 void ozaki_gemm(Ctx& c, const OzProblem* d_probs, const int* d_tiles, int ntiles, int* d_status) {
     if (ntiles == 0) return;
     // the limit is per device: set it on every launch
     RA_CUDA(cudaFuncSetAttribute(ozaki_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OzSmem)));
-    const int grid = std::min(ntiles, oz_sm_count());
+    const int grid = std::min(ntiles, sm_count());
     ozaki_gemm_kernel<<<grid, OZ_THREADS, sizeof(OzSmem), c.stream>>>(
         d_probs, reinterpret_cast<const int4*>(d_tiles), ntiles, d_status);
     RA_CUDA(cudaGetLastError());

@@ -36,46 +36,49 @@ __device__ __forceinline__ double2 twiddle(const double2* wr, int N, int e, int 
     return w;
 }
 
-// Runs nb independent FFTs of length N stored at a + b*N (b < nb), scratch at
-// bb + b*N; returns the buffer base holding the results.  Must be entered with
-// a synchronised input; leaves the result synchronised.
-__device__ double2* fft_run(double2* a, double2* bb, int nb, const FFTPlan& pl, const double2* wr, int sign) {
-    const int N = pl.n;
-    int p = 1;
-    double2* src = a;
-    double2* dst = bb;
-    for (int ps = 0; ps < pl.npass; ++ps) {
-        const int R = pl.radix[ps];
-        const int T = N / R;
-        const int stride = N / (p * R);
-        for (int g = threadIdx.x; g < T * nb; g += blockDim.x) {
-            const int b = g / T, bi = g - b * T;
-            const double2* sb = src + b * N;
-            double2* db = dst + b * N;
-            const int k = bi % p;
-            double2 u[8];
+// One pass of radix R of the FFT of length N in src, to dst; p is the product of the radices before.
+template <int R>
+__device__ __forceinline__ void fft_run_pass(const double2* __restrict__ src, double2* __restrict__ dst, int N, int p,
+                                             const double2* wr, int sign) {
+    const int T = N / R, stride = N / (p * R);
+    for (int g = threadIdx.x; g < T; g += blockDim.x) {
+        const int k = g % p;
+        double2 u[R];
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
-                if (r < R) u[r] = sb[bi + r * T];
+        for (int r = 0; r < R; ++r) u[r] = src[g + r * T];
 #pragma unroll
-            for (int r = 1; r < 8; ++r)
-                if (r < R) u[r] = cmul(u[r], twiddle(wr, N, r * k * stride, sign));
-            dft_small(R, u, sign);
-            const int j = (bi - k) * R + k;
+        for (int r = 1; r < R; ++r) u[r] = cmul(u[r], twiddle(wr, N, r * k * stride, sign));
+        dft_small(R, u, sign);
+        const int j = (g - k) * R + k;
 #pragma unroll
-            for (int r = 0; r < 8; ++r)
-                if (r < R) db[j + r * p] = u[r];
-        }
-        __syncthreads();
-        double2* t = src;
-        src = dst;
-        dst = t;
-        p *= R;
+        for (int r = 0; r < R; ++r) dst[j + r * p] = u[r];
     }
-    return src;
 }
 
-// ---- compile-time plans of the in-place FFT: greedy radix order 16, 8, 4, 2, 3 ----
+// Runs the FFT of length N in a, scratch in b; returns the buffer holding the result.  Must be entered
+// with a synchronised input; leaves the result synchronised.
+__device__ double2* fft_run(double2* a, double2* b, const FFTPlan& pl, const double2* wr, int sign) {
+    int p = 1;
+    for (int ps = 0; ps < pl.npass; ++ps) {
+        const int R = pl.radix[ps];
+        if (R == 8)
+            fft_run_pass<8>(a, b, pl.n, p, wr, sign);
+        else if (R == 4)
+            fft_run_pass<4>(a, b, pl.n, p, wr, sign);
+        else if (R == 2)
+            fft_run_pass<2>(a, b, pl.n, p, wr, sign);
+        else
+            fft_run_pass<3>(a, b, pl.n, p, wr, sign);
+        __syncthreads();
+        double2* t = a;
+        a = b;
+        b = t;
+        p *= R;
+    }
+    return a;
+}
+
+// ---- compile-time plans of the in-place FFT: greedy radix order 8, 4, 2, 3 ----
 __host__ __device__ constexpr int radix_at(int n, int i) {
     int m = n, k = 0;
     while (m % 8 == 0) { if (k == i) return 8; m /= 8; ++k; }
@@ -106,24 +109,12 @@ __device__ __forceinline__ int SW(int i) { return i; }
 // eight different bank groups per quarter warp (n is a multiple of 8).
 __host__ __device__ constexpr int fstride(int n) { return n + 2; }
 
-// One CTA = one (theta, r) row; the rows theta and pi - theta of a pair form a
-// 2-CTA cluster that folds its spectra through distributed shared memory.
 // Threads of a row CTA: half a thread per complex point, whole warps, at most 384.  The diagnostics
 // transform one or a few fields at a time, N / 8 butterflies a pass: with 384 threads at every N most
 // of them waited at the barriers of a small row, and few rows fitted an SM (n_theta = 192, N_r = 64:
 // shell averages of seven quantities 6.5 -> 2.2 ms, azimuthal 3.5 -> 1.4, global 3.4 -> 1.3).
 __host__ __device__ constexpr int row_threads(int n) { return n >= 768 ? 384 : (n / 2 + 31) / 32 * 32; }
 constexpr int FB = 4;   // fields per batched FFT
-
-// Shared memory of a row CTA (double2 units): one in-place FFT buffer of FB
-// fields and the four nonlinear outputs (W, P, T, Z; each thread owns its
-// points; the r2c runs in place on them).
-template <int N>
-struct RowSmem {
-    static constexpr int FS = fstride(N);
-    static constexpr int BUF = 0, ACC = FB * FS;
-    static constexpr int SIZE = ACC + 4 * FS;
-};
 
 // In-place mixed-radix FFT passes (field f at f*FS).  Pass s:
 // sub-transform length LS = N / (R_0 ... R_{s-1}), radix R = R_s, stride
@@ -241,9 +232,8 @@ __device__ __forceinline__ void fft_pass_ip(double2* __restrict__ buf, const dou
 #pragma unroll
         for (int m = 0; m < R; ++m) buf[SW(base + m * SS)] = u[m];
     };
-    // two independent butterflies per iteration for instruction-level parallelism
-    // (one for radix 16, whose butterfly alone fills the registers)
-    if constexpr (R >= 16 || NT > 256) {
+    // two independent butterflies per iteration for instruction-level parallelism, one in the rows of 384 threads
+    if constexpr (NT > 256) {
 #pragma unroll 1
         for (int g = tid; g < T * NB; g += NT) butterfly(g);
     } else {
@@ -319,7 +309,7 @@ __device__ __forceinline__ void row_c2r(const PhysParams& P, const double* __res
     constexpr int FS = fstride(N);
     constexpr int NI = N / 2 + 1;                                   // k = 0 .. N/2
     constexpr int QI = (NB * NI + row_threads(N) - 1) / row_threads(N);   // items per thread
-    double2* buf = sm + RowSmem<N>::BUF;
+    double2* buf = sm;
     const int L = P.L;
     const long ostride = (long)P.ncola;   // E -> O within p2a[theta_h][m][par][r][field][2]
     const long mstride = 2L * P.ncola;
@@ -779,7 +769,12 @@ void launch_physics(Ctx& c) {
     launch_physics_pair(c, P);
 }
 
-__global__ void fft_rows_kernel(double* x, long howmany, const double2* wrg, FFTPlan plan, int inverse) {
+// The packed real FFT of single rows in place: one CTA a row, two row buffers and the twiddles in shared
+// memory.  CTAS: registers for that many CTAs an SM.  Four (64 registers) hide each other's barriers best
+// (n_theta 384, 256 columns, c2r: 1.00 ms, with three and 72 registers 1.19); three where the shared
+// memory, 48 bytes a point, holds no more (n_theta 1536, 64 columns: 3.21 ms, with 64 registers 3.33).
+template <int CTAS>
+__global__ void __launch_bounds__(256, CTAS) fft_rows_kernel(double* x, long howmany, const double2* wrg, FFTPlan plan, int inverse) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int N = plan.n;
     double2* a = reinterpret_cast<double2*>(smem_raw);
@@ -800,7 +795,7 @@ __global__ void fft_rows_kernel(double* x, long howmany, const double2* wrg, FFT
             a[k] = make_double2(e.x - wd.y, e.y + wd.x);
         }
         __syncthreads();
-        double2* res = fft_run(a, b, 1, plan, wr, +1);
+        double2* res = fft_run(a, b, plan, wr, +1);
         for (int n = threadIdx.x; n < N; n += blockDim.x) {
             row[2 * n] = res[n].x;
             row[2 * n + 1] = res[n].y;
@@ -810,7 +805,7 @@ __global__ void fft_rows_kernel(double* x, long howmany, const double2* wrg, FFT
     } else {
         for (int n = threadIdx.x; n < N; n += blockDim.x) a[n] = make_double2(row[2 * n], row[2 * n + 1]);
         __syncthreads();
-        double2* Z = fft_run(a, b, 1, plan, wr, -1);
+        double2* Z = fft_run(a, b, plan, wr, -1);
         for (int k = threadIdx.x; k <= N; k += blockDim.x) {
             const double2 zk = Z[k % N];
             const double2 zn = cconj(Z[(N - k) % N]);
@@ -829,9 +824,15 @@ __global__ void fft_rows_kernel(double* x, long howmany, const double2* wrg, FFT
 void launch_fft_rows(Ctx& c, double* d_x, long howmany, int inverse) {
     FFTPlan plan = make_plan(c.d.nth);
     const size_t smem = 3 * (size_t)c.d.nth * sizeof(double2);
-    allow_shared(fft_rows_kernel);
-    fft_rows_kernel<<<(unsigned)howmany, 256, smem, c.stream>>>(d_x, howmany, reinterpret_cast<const double2*>(c.d_twid),
-                                                              plan, inverse);
+    auto go = [&](auto kern) {
+        allow_shared(kern);
+        kern<<<(unsigned)howmany, 256, smem, c.stream>>>(d_x, howmany, reinterpret_cast<const double2*>(c.d_twid), plan,
+                                                         inverse);
+    };
+    if (4 * smem <= (size_t)SMEM_BLOCK)
+        go(fft_rows_kernel<4>);
+    else
+        go(fft_rows_kernel<3>);
     RA_CUDA(cudaGetLastError());
     ++c.launches;
 }
@@ -1393,7 +1394,7 @@ void launch_spectra_rows(Ctx& c, const SliceSpec& S, int slot0, double* p2b) {
 
 void launch_spectra_gather(Ctx& c, const double* s2, int nslots, double* out) {
     const long total = (long)nslots * 2 * c.d.L * c.d.L;
-    const unsigned blocks = (unsigned)std::min<long>((total + 255) / 256, 148L * 16);
+    const unsigned blocks = (unsigned)std::min<long>((total + 255) / 256, 16L * sm_count());
     spectra_gather_kernel<<<blocks, 256, 0, c.stream>>>(s2, c.d.L, nslots, (long)c.nfb * c.d.nr * 2, out);
     RA_CUDA(cudaGetLastError());
     ++c.launches;

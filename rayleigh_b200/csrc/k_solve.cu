@@ -817,7 +817,7 @@ void solve_prepare(Ctx& c) {
     // (l_max 41, N_r 48: 33 -> 25 us; at l_max 63, 160 tiles, 48 -> 51 us, at 127 138 -> 167 us).
     long tiles = 0;
     for (int l = 0; l < c.d.L; ++l) tiles += (2 * (l + 1) + 31) / 32;
-    if (tiles <= 148) c.solve_nc = c.solve_nc_z = 16;
+    if (tiles <= sm_count()) c.solve_nc = c.solve_nc_z = 16;
     rebuild_solve_tiles(c);
 }
 

@@ -245,7 +245,7 @@ void launch_cheb_synthesis(Ctx& c) {
     // Where the (tile, field) CTAs leave SMs without three of them, the derivative orders go to CTAs of
     // their own: the chain of up to four orders is what a small grid waits for.
     dim3 grid((unsigned)((ncols + CH_COLS - 1) / CH_COLS), c.mag ? 6 : 4);
-    if (grid.x * grid.y < 3 * 148) grid.z = 4;
+    if (grid.x * grid.y < 3u * sm_count()) grid.z = 4;
     cheb_synthesis_kernel<<<grid, CH_THREADS, smem, c.stream>>>(c.d_D, c.d_sol_wpt, c.d_sol_z, c.d_sol_c, c.d_sol_a,
                                                                 c.d_g, c.d.nr, c.d.kc, ncols);
     RA_CUDA(cudaGetLastError());

@@ -946,7 +946,7 @@ static void release(Ctx& c) {
                       c.d_xemf, c.d_Memf, c.d_Ainv_c, c.d_Ainv_a};
     for (double* b : bufs)
         if (b) cudaFree(b);
-    int* ibufs[] = {c.d_ltiles, c.d_inv_tiles, c.d_fwd_tiles, c.d_cheb_tiles, c.d_solve_tiles, c.d_status,
+    int* ibufs[] = {c.d_fwd_tiles, c.d_solve_tiles, c.d_status,
                     c.d_perm_wpt, c.d_perm_z, c.d_skip_z, c.d_inv_sol_tiles, c.d_inv_sol_tiles_z,
                     c.d_perm_c, c.d_perm_a};
     for (int* b : ibufs)

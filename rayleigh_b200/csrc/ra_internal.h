@@ -201,9 +201,8 @@ struct Ctx {
     int solve_nc = 32, solve_nc_z = 32;               // right-hand-side columns per substitution CTA (W-P-T, Z)
     int n_inv_sol_tiles = 0, n_inv_sol_tiles_z = 0, n_solve_tiles_z = 0;
     int *d_inv_sol_tiles = nullptr, *d_inv_sol_tiles_z = nullptr;   // tile lists of the explicit inverses (mixed form)
-    int *d_ltiles = nullptr;                          // LT tile lists
-    int n_inv_tiles = 0, n_fwd_tiles = 0, n_cheb_tiles = 0, n_solve_tiles = 0;
-    int *d_inv_tiles = nullptr, *d_fwd_tiles = nullptr, *d_cheb_tiles = nullptr, *d_solve_tiles = nullptr;
+    int n_fwd_tiles = 0, n_solve_tiles = 0;
+    int *d_fwd_tiles = nullptr, *d_solve_tiles = nullptr;   // tile lists of the forward Legendre product and the solves
 
     // device state and step buffers
     double *d_sol_wpt = nullptr, *d_sol_z = nullptr;  // [lm][2][3nr], [lm][2][nr]
@@ -374,6 +373,14 @@ inline void allow_shared(F* kern) {
     cudaFuncAttributes a;
     RA_CUDA(cudaFuncGetAttributes(&a, kern));
     RA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BLOCK - (int)a.sharedSizeBytes));
+}
+
+// SMs of the current device (asked on every call: one process may drive several devices)
+inline int sm_count() {
+    int dev = 0, n = 0;
+    RA_CUDA(cudaGetDevice(&dev));
+    RA_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    return n;
 }
 
 struct SingularError {   // a zero pivot in a per-l matrix: RA_ERR_SINGULAR
