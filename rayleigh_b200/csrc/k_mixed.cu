@@ -58,8 +58,11 @@ static void run_split_once(Ctx& c, const std::vector<OzSplitJob>& jobs, int max_
 // ---------------------------------------------------------------------------
 // Whether the mixed form's Legendre products are split products.  On small grids the digit split and
 // the product's short K cost more than the FP64 products, which are the more exact anyway: per step
-// at N_r = 64 with B, FP64 / split, the inverse takes 51 / 115 us at l_max = 63, 250 / 301 at 127 and
-// 441 / 610 at 170, but 1263 / 1009 at 255; the forward 35 / 67, 113 / 147, 230 / 209 and 598 / 423.
+// at N_r = 64 with B, FP64 / split, the inverse takes 43 / 116 us at l_max = 63, 345 / 613 at 170,
+// 1014 / 1011 at 255 and 2258 / 1723 at 340; the forward 32 / 65, 205 / 210, 536 / 420 and 1163 / 735.
+// The line depends on l_max alone: batches of 1 to 2048 columns (l_max 147 to 201) are never slower in FP64
+// below it, by 1.15 (inverse, l_max 198, 2048 columns) to 3 times (one column), the forward by 1.05 and more.
+// Between 199 and 255 the inverse is about even (l_max 201, 512 columns 325 / 385 us, l_max 255 477 / 497).
 bool lt_split(const Ctx& c, bool inverse) { return c.d.L >= (inverse ? 200 : 150); }
 
 // The plan of one batched inverse transform p2 = P s2 over ncol columns (s2 rows in the

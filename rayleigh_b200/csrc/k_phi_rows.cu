@@ -5,10 +5,12 @@
 //   rows_r2c  rows -> their packed spectra in place, and the folded p2[m][par][theta_h][fr]
 // on row pairs (phi_pair.cuh), four neighbouring columns fr per T = n_phi / 4 threads.
 //
-// What bounds them: HBM.  Each direction reads its input once and writes its output once, where
-// the separate relayout and in-place FFT moved the rows three times and the FFT, one row per CTA
-// with a twiddle table copied to shared memory for each, ran at a fifth of the HBM rate (l_max 255, 512
-// columns, FP64 inverse call: 3303 -> 1130 us).
+// What bounds them: latency.  At n_phi = 1536 registers let one CTA of twelve warps on an SM, which waits
+// on its loads (long scoreboard a third of the cycles of an instruction) and barriers; the L1 data pipe is
+// 59 % busy, HBM 0.37 (c2r) and 0.56 (r2c, whose rows' spectra are 37 % of its bytes) of the copy rate.  Each
+// direction reads its input once and writes its output once, where the separate relayout and in-place FFT moved
+// the rows three times and the FFT, one row per CTA with a twiddle table copied to shared memory for each, ran
+// at a fifth of the HBM rate (l_max 255, 512 columns, FP64 inverse call: 3303 -> 1130 us).
 // The rows enter and leave in natural phi order: the points of the last pass, digit-reversed, go
 // through shared memory once more, at natural index n plus one slot per F R1 points, which
 // spreads the 8 lanes of a phase (their n differ by F R1) over the 8 banks.

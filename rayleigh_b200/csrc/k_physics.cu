@@ -405,8 +405,8 @@ void physics_prepare(Ctx& c) {
     }
     physics_pair_prepare(c);
     c.physics3_ok = p3_supported(c.d.nth);
-    // default: the row-pair kernel where it exists (l_max = 511, N_r = 96 with B: 12.6 ms against
-    // 16.6 ms of one CTA per row); the autotuner measures the others too
+    // default: the row-pair kernel where it exists (k_physics_pair.cu has the times of both); the autotuner
+    // measures the others too
     c.physics_form = physics_pair_supported(c.d.nth) ? 1 : 0;
     if (!c.physics3_ok && !physics_pair_supported(c.d.nth))
         throw ArgError("n_theta " + std::to_string(c.d.nth) + " has no physical-space kernel instance");

@@ -12,10 +12,14 @@
 // The transform and its layout: phi_pair.cuh.
 //
 // What bounds it: at most twelve warps an SM (168 registers hold the velocity or B and a batch's
-// points, 8 M slots of shared memory a batch and the four outputs), which wait in turn on loads,
-// barriers and shared memory; the data pipe is 68 % busy at M = 1536.  Against one CTA of 384 threads
-// per row with half-length transforms, per step: n_theta 64, N_r 48 127.6 -> 31 us; 192 polytrope,
-// N_r 128 1331 -> 588; 384 anelastic MHD, N_r 128 6751 -> 3811; 768 dynamo, N_r 96 16.56 -> 12.35 ms.
+// points, 8 M slots of shared memory a batch and the four outputs; at M = 1024 eight, the shared memory of
+// one CTA of 256 threads, which take 238 to 255 registers), which wait in turn on loads, barriers and shared
+// memory; the data pipe is 68 % busy at M = 1536.  Against one CTA of 384 threads per row with
+// half-length transforms, per step: n_theta 64, N_r 48 127.6 -> 31 us; 192 polytrope, N_r 128 1331 -> 588;
+// 384 anelastic MHD, N_r 128 6751 -> 3811; 512, N_r 64 hydrodynamic 4.73 -> 2.51 ms, dynamo 7.31 -> 3.82,
+// anelastic MHD 7.53 -> 3.99; 768 dynamo, N_r 96 16.56 -> 12.4.  At M = 1536 the heating terms spill (384 bytes
+// without B, 228 with): 768, N_r 64 polytrope 7.45 -> 6.03 ms, anelastic MHD 11.60 -> 9.31, against
+// 5.62 and 8.30 without heating.
 #include <cmath>
 #include <vector>
 
@@ -86,7 +90,7 @@ __global__ void __launch_bounds__(G* M / 4, MINB) physics_pair_kernel(PhysParams
     constexpr int T = Pair<M>::T, NT = G * T, NTH = M / 2;
     // The next batch's spectra come in under this one's terms, except in the largest plans (two radix-8
     // mid passes): with both the staging and up to six transforms inlined their code outgrows the
-    // instruction cache (M = 1536 with B, N_r = 96: 16.2 ms staged, 12.3 direct; M = 768 with B and
+    // instruction cache (M = 1536 with B, N_r = 96: 16.2 ms staged, 12.4 direct; M = 768 with B and
     // heating, N_r = 128: 3.81 / 3.83 ms, M = 384 with heating 588 / 667 us, with B, N_r = 64,
     // 451 / 515, M = 256 195 / 218).
     constexpr bool STAGED = Pair<M>::R1 < 8;

@@ -104,7 +104,7 @@ def test_fd_step_rate():
     """The finite-difference step against the Chebyshev step on one grid (Boussinesq
     hydrodynamic, N_r = 128, l_max = 255, N_theta = 384), FP64 and mixed: steps/s over 50
     graph-replayed steps, host-timed between two state copies; prints the four rates
-    (measured: Chebyshev 81.1 / 97.5, finite differences 79.7 / 81.7 steps/s FP64 / mixed; the
+    (measured: Chebyshev 106.3 / 120.4, finite differences 106.0 / 103.8 steps/s FP64 / mixed; the
     finite-difference mixed form solves by the FP64 substitution)."""
     import time
     cfg = dict(n_r=128, l_max=255, dt=1e-6, rayleigh=1e5, ekman=1e-3, use_graph=True)

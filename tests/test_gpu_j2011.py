@@ -84,7 +84,7 @@ def test_j2011_hydro_steady_solution():
     means = {k: float(np.mean(v)) for k, v in samples.items()}
     diff = {k: 100.0 * (means[k] - GOLD["suggested"][k]) / abs(GOLD["suggested"][k]) for k in means}
     print(f"j2011 hydro: {time.time() - t0:.0f} s, {changes} dt changes; means {means}; % difference {diff}")
-    # measured (FP64, 200000 steps of 30 s in 559 s on one B200): KE -0.011 %, zonal KE -0.014 %,
+    # measured (FP64, 200000 steps of 30 s in 329 s on one B200): KE -0.011 %, zonal KE -0.014 %,
     # meridional KE -0.018 %, entropy -0.004 %, v_phi -0.56 % from the suggested values
     bounds = {"Kinetic Energy": 0.1, "Zonal KE": 0.1, "Meridional KE": 0.1, "Entropy": 0.05, "Vphi": 1.0}
     for k, b in bounds.items():
