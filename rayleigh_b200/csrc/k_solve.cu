@@ -813,8 +813,10 @@ static T* upload_vec(Ctx& c, const std::vector<T>& v) {
 void solve_prepare(Ctx& c) {
     c.solve_nc = lu_nc_for(3 * c.d.nr);
     c.solve_nc_z = lu_nc_for(c.d.nr);
-    // Fewer tiles than SMs: narrower ones fill more of them, and a CTA's chain of products halves
-    // (l_max 41, N_r 48: 33 -> 25 us; at l_max 63, 160 tiles, 48 -> 51 us, at 127 138 -> 167 us).
+    // Fewer tiles than SMs: narrower ones fill more of them, and a CTA's chain of products halves: faster or
+    // even at n_theta 24 to 64 for every N_r from 16 to 192, with and without B (l_max 41: N_r 48 32.6 -> 25.9 us,
+    // with B 35.9 -> 32.4; N_r 192 208 -> 161).  Above the line it depends on the systems (l_max 63, 160 tiles,
+    // N_r 64 47.6 -> 41.1 us, with B 49.9 -> 55.0; l_max 127, N_r 64 with B 138 -> 167).
     long tiles = 0;
     for (int l = 0; l < c.d.L; ++l) tiles += (2 * (l + 1) + 31) / 32;
     if (tiles <= sm_count()) c.solve_nc = c.solve_nc_z = 16;
